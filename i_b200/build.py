@@ -1,4 +1,4 @@
-"""Builds libi_core.so (the C++ core plus the sm_100a kernels) in-tree.
+"""Builds libi_core.so (the C++ core plus the sm_100a kernels) and the Python call modules in-tree.
 
 Every translation unit is compiled with
 `nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo -O3` and linked with the
@@ -6,7 +6,9 @@ static CUDA runtime, so the library loads on a machine without a GPU or driver
 (calls that need a device then fail with an error message).  Run as
 `python -m i_b200.build` or through `__graft_entry__.build()`.
 """
+import importlib.util
 import os
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -82,6 +84,31 @@ def _compile(src, headers, verbose, obj_dir=None, extra=()):
     return obj, proc.stderr if verbose else ""
 
 
+def _build_call_modules(out_dir):
+    """The extension modules ilang.py marshals its calls through (csrc/python): NumPy arrays with
+    Python's C API alone, CUDA tensors with torch's headers and libraries."""
+    import sysconfig
+    common = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-I", os.path.join(REPO, "include"),
+              "-isystem", sysconfig.get_paths()["include"]]
+    jobs = {"host_call": []}
+    spec = importlib.util.find_spec("torch")
+    if spec is not None and spec.submodule_search_locations:
+        torch_dir = list(spec.submodule_search_locations)[0]
+        inc, lib = os.path.join(torch_dir, "include"), os.path.join(torch_dir, "lib")
+        cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(_nvcc()) or _nvcc()))),
+                            "include")
+        jobs["cuda_call"] = ["-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
+                             "-isystem", cuda, "-L", lib, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    for name, extra in jobs.items():
+        src = os.path.join(CSRC, "python", name + ".cc")
+        out = os.path.join(out_dir, "_%s.so" % name)
+        if _newer(out, [src] + _headers()):
+            continue
+        proc = subprocess.run(common + [src, "-o", out] + extra, capture_output=True, text=True)
+        if proc.returncode != 0:
+            raise RuntimeError("g++ failed for %s:\n%s" % (src, proc.stderr))
+
+
 def build(verbose=False, force=False, out_dir=None, extra_flags=()):
     """Compile what changed and link libi_core.so; returns its path.
 
@@ -108,6 +135,7 @@ def build(verbose=False, force=False, out_dir=None, extra_flags=()):
         proc = subprocess.run(cmd, capture_output=True, text=True)
         if proc.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (proc.stdout, proc.stderr))
+    _build_call_modules(out_dir)
     return lib
 
 

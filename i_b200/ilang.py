@@ -21,7 +21,10 @@ no usable GPU every exec raises RuntimeError with the runtime's message.
 """
 import array
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
+import sys
 import weakref
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -108,6 +111,35 @@ def launch_count():
 def set_reserved_sms(n):
     """Leave n SMs free next to the persistent attention kernel (for collectives)."""
     _ok(_core.i_b200_set_reserved_sms(int(n)))
+
+
+# Native marshalling of the common calls (csrc/python): {kind: module}, None where it cannot be used.
+_native = {}
+
+
+def _native_call(kind):
+    """The extension module that makes calls with CUDA tensors ("cuda") or NumPy arrays ("host")
+    without ctypes, or None.  Loaded on first use, and only once torch (or NumPy) is in the process."""
+    needs = {"cuda": "torch", "host": "numpy"}[kind]
+    if kind not in _native:
+        if needs not in sys.modules:
+            return None
+        module = None
+        path = os.path.join(_HERE, "lib", "_%s_call.so" % kind)
+        if os.path.exists(path):
+            name = "_%s_call" % kind
+            loader = importlib.machinery.ExtensionFileLoader(name, path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
+            loader.exec_module(module)
+            symbols = ["i_b200_exec_into" if kind == "cuda" else "i_exec_into", "i_output_count",
+                       "i_output_ranks", "i_output_shapes", "i_error"]
+            addresses = [ctypes.cast(getattr(_core, s), _VOIDP).value for s in symbols]
+            if kind == "host":
+                import numpy as np
+                addresses += [np.ndarray, np.empty, np.float32]
+            module.bind(*addresses)
+        _native[kind] = module
+    return _native[kind]
 
 
 def _fail():
@@ -377,10 +409,20 @@ class Component:
 
     def exec_numpy(self, *inputs):
         import numpy as np
+        native = _native.get("host") or _native_call("host")
+        if native is not None:
+            done = native.exec(self._compiled[0] or self._compile(), inputs)
+            if done is not None:
+                return done
         return self._run_into_new(lambda shape: np.empty(shape, dtype=np.float32), inputs)
 
     def exec_torch(self, *inputs):
         import torch
+        native = _native.get("cuda") or _native_call("cuda")
+        if native is not None:
+            done = native.exec(self._compiled[0] or self._compile(), inputs)
+            if done is not None:
+                return done
         device = next((x.device for x in inputs if _on_cuda(x)), "cpu")
         return self._run_into_new(lambda shape: torch.empty(shape, dtype=torch.float32, device=device),
                                   inputs)
@@ -395,7 +437,13 @@ class Component:
         torch's current stream is synchronised first: the runtime's own stream is
         not ordered behind work that is still producing them.
         """
-        program = self._compile()
+        program = self._compiled[0] or self._compile()
+        for kind in ("cuda", "host"):
+            native = _native.get(kind) or _native_call(kind)
+            if native is not None:
+                done = native.into(program, outputs, inputs)
+                if done is not None:
+                    return done
         single = not isinstance(outputs, (tuple, list))
         if single:
             outputs = (outputs,)
