@@ -34,6 +34,7 @@ SOURCES = [
     "kernels/device_util.cu",
     "kernels/gemm_tcgen05.cu",
     "kernels/attention_tcgen05.cu",
+    "kernels/attention_direct.cu",
     "kernels/dispatch.cu",
     "kernels/attention_static.cu",
 ]

@@ -52,10 +52,12 @@ void* scratch_on_current_device() {
 extern "C" int ib_attention_static(const float* q, const float* k, const float* v, float* o,
                                    size_t batch, size_t nq, size_t nk, size_t d, size_t dv,
                                    int v_kmajor, void* stream) {
-  const size_t need =
-      ib_attention_workspace_bytes(batch, nq, nk, d, dv, v_kmajor, IB_PRECISION_FP32);
+  size_t need = ib_attention_workspace_bytes(batch, nq, nk, d, dv, v_kmajor, IB_PRECISION_FP32);
   if (need == SIZE_MAX)
     return ib::fail("ib_attention_static: extents too large (an element count does not fit size_t)");
+  // The documented limit is the score matrix, also where the kernel behind the call keeps none.
+  const size_t scores = (batch * nq * nk * sizeof(float) + 255) / 256 * 256;
+  if (need < scores) need = scores;
   if (need > kStaticScratchBytes)
     return ib::fail("ib_attention_static: batch*nq*nk = " + std::to_string(batch * nq * nk) +
                     " scores need " + std::to_string(need) + " bytes of scratch, the built-in " +

@@ -85,6 +85,21 @@ bool attention_shape_ok(size_t d, size_t dv) {
   return d % 4 == 0 && d >= 4 && d <= 128 && dv >= 1 && dv <= 128;
 }
 
+// Attention straight from K and V in fp32 (attention_direct.cu).  Two rules:
+//   up to kDirectQueries queries per head, under every precision: the pass is then bound by reading K
+//   and V once, which the tensor arms cannot do (they first write converted copies of both, as many
+//   bytes again), and no arm is less exact;
+//   otherwise fp32 arithmetic up to kDirectFlop: above that two tiled contractions with the scores in
+//   memory between them are faster.
+constexpr size_t kDirectQueries = 8;
+constexpr double kDirectFlop = 1073741824.0;    // 2^30
+bool attention_prefers_direct(size_t batch, size_t nq, size_t nk, size_t d, size_t dv, bool v_kmajor, int precision) {
+  if (v_kmajor || !attention_direct_shape_ok(batch, nq, nk, d, dv)) return false;
+  if (nq <= kDirectQueries) return true;
+  const double flop = 4.0 * batch * nq * nk * d;
+  return !wants_tensor(precision, flop) && flop <= kDirectFlop;
+}
+
 // Which arithmetic the fused attention kernel uses for a precision request: AUTO and F16 take the
 // fp16 arm (both contractions on fp16 operands scaled into range: TF32's mantissa, half the
 // tensor-core instructions), TF32_F16 the mixed arm (TF32 for Q K^T, fp16 for P V), TF32 the pure
@@ -554,6 +569,8 @@ extern "C" size_t ib_attention_workspace_bytes(size_t batch, size_t nq, size_t n
   if (too_many_elements({batch, nq, nk}) || too_many_elements({batch, nq, d > dv ? d : dv}) ||
       too_many_elements({batch, nk, d > dv ? d : dv}))
     return SIZE_MAX;
+  if (attention_prefers_direct(batch, nq, nk, d, dv, v_kmajor != 0, precision))
+    return carve_bytes(attention_direct_floats(batch, nq, nk, dv));
   const double flop = 4.0 * batch * nq * nk * d;
   if (wants_tensor(precision, flop) && attention_shape_ok(d, dv)) {
     // Rounded copy of K, V^T (rounded), and the KV-split partials; bf16 copies
@@ -588,6 +605,14 @@ extern "C" int ib_attention_scaled(const float* q, const float* k, const float* 
   Carver ws(workspace, workspace_bytes);
   const double flop = 4.0 * batch * nq * nk * d;
   const bool tensor = wants_tensor(precision, flop);
+
+  if (attention_prefers_direct(batch, nq, nk, d, dv, v_kmajor != 0, precision)) {
+    const size_t floats = attention_direct_floats(batch, nq, nk, dv);
+    float* partials = floats ? ws.take(floats) : nullptr;
+    if (floats && !partials)
+      return fail("ib_attention: workspace too small (see ib_attention_workspace_bytes)");
+    return attention_direct(q, k, v, o, batch, nq, nk, d, dv, logit_scale, logit_divide != 0, partials, s);
+  }
 
   if (tensor && attention_shape_ok(d, dv)) {
     PreparedKV kv;

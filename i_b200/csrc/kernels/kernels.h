@@ -154,6 +154,15 @@ int prepare_attention_operands_bf16(const float* k, void* k16, const float* v, v
                                     size_t batch, size_t nk, size_t d, size_t dv, size_t d_pitch,
                                     size_t nk_pitch, bool v_kmajor, cudaStream_t s);
 
+// attention_direct.cu — the same attention in fp32, straight from the caller's arrays (V as [nk][dv]):
+// few queries per head or small problems.  `partials` holds attention_direct_floats floats (8-byte
+// aligned; null when that is 0).
+bool attention_direct_shape_ok(size_t batch, size_t nq, size_t nk, size_t d, size_t dv);
+size_t attention_direct_floats(size_t batch, size_t nq, size_t nk, size_t dv);
+int attention_direct(const float* q, const float* k, const float* v, float* o, size_t batch, size_t nq,
+                     size_t nk, size_t d, size_t dv, const float* logit_scale, bool logit_divide,
+                     float* partials, cudaStream_t s);
+
 void set_attention_profile(unsigned long long* device_counters);
 void set_reserved_sms(int n);
 int reserved_sms();

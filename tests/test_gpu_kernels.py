@@ -920,3 +920,30 @@ def test_attention_many_row_blocks_of_few_key_tiles(lib, torch, batch, nq, nk, p
     ref = torch.softmax(q @ k.transpose(1, 2), dim=-1) @ v
     assert torch.isfinite(o).all()
     assert ((o - ref).abs().max() / ref.abs().max()).item() <= tol
+
+
+@pytest.mark.parametrize("batch,nq,nk,d,dv", [
+    (1, 1, 1, 1, 1), (2, 2, 31, 4, 3), (3, 3, 33, 32, 32),      # a block of 32 keys and its edges, 8 lanes a key
+    (1, 1, 9000, 128, 128), (5, 2, 6000, 128, 100),             # key ranges merged by a second kernel
+    (40, 1, 2500, 128, 128), (20, 4, 1300, 64, 48),             # ... in a cluster
+    (2, 9, 257, 36, 65), (1, 128, 128, 64, 64), (3, 300, 511, 128, 128), (1, 7, 100, 33, 127)])
+@pytest.mark.parametrize("scale", [None, 0.3, -4.0])
+def test_attention_direct_fp32(lib, torch, batch, nq, nk, d, dv, scale):
+    # The one-pass fp32 kernel: 1 to 8 queries a warp, 8 to 32 lanes a key, one to many key ranges.  fp32
+    # products and sums: a few hundred roundings of 2^-24 on probabilities and on V, 1e-5 of the peak.
+    q, k, v = rand((batch, nq, d), 91), rand((batch, nk, d), 92), rand((batch, nk, dv), 93)
+    q *= np.float32(d ** -0.5)
+    sc = None if scale is None else torch.tensor(scale, device="cuda", dtype=torch.float32)
+    ws_bytes = lib.ib_attention_workspace_bytes(batch, nq, nk, d, dv, 0, FP32)
+    ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device="cuda")
+    out = torch.full((batch, nq, dv), float("nan"), device="cuda")
+    dq, dk, dv_ = dev(torch, q), dev(torch, k), dev(torch, v)
+    ok(lib, lib.ib_attention_scaled(dq.data_ptr(), dk.data_ptr(), dv_.data_ptr(), out.data_ptr(), batch, nq, nk, d,
+                                    dv, 0, FP32, 0, None if sc is None else sc.data_ptr(), int(scale == -4.0),
+                                    ws.data_ptr(), ws_bytes, None))
+    s = np.einsum("bqd,bkd->bqk", q.astype(np.float64), k.astype(np.float64))
+    if scale is not None:
+        s = s / np.float64(np.float32(scale)) if scale == -4.0 else s * np.float64(np.float32(scale))
+    p = np.exp(s - s.max(axis=2, keepdims=True))
+    want = np.einsum("bqk,bkv->bqv", p / p.sum(axis=2, keepdims=True), v.astype(np.float64))
+    assert max_rel_to_peak(out.cpu().numpy(), want) <= TOL_FP32
