@@ -59,6 +59,29 @@ __device__ __forceinline__ float weight_of(float x, float m) {
   return exp_e32_fast(x - (m == -CUDART_INF_F ? 0.0f : m));
 }
 
+// Two products or multiply-adds in one instruction, each lane rounded as the plain one.
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t pack(float lo, float hi) {
+  pair_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack(pair_t x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+__device__ __forceinline__ pair_t mul2(pair_t a, pair_t b) {
+  pair_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
+  pair_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // Sums v[0..7] across the LP lanes of a key row.  Lane `sub` returns the sum of v[sub / (LP / 8)].
 template <int LP>
 __device__ __forceinline__ float sum_eight(float (&v)[8], int sub) {
@@ -84,7 +107,14 @@ attention_direct_kernel(DirectArgs a) {
   constexpr int kKeysPerLoad = 32 / LP;
   constexpr int kBatches = LP / 8;           // of eight loads: together one block of 32 keys
   constexpr int kWidth = LP * 4;             // features a warp covers
-  __shared__ float sm_o[kWarps][NQ][kWidth];
+  // With four or eight queries the registers are the accumulators': the queries stay in shared
+  // memory (one 16-byte read per eight rows and query), and a weight reaches the lanes as a
+  // duplicated pair from shared memory (a 16-byte broadcast for two queries, where a shuffle serves one).
+  constexpr bool kWide = NQ >= 4;
+  constexpr int kBatchUnroll = kWide ? 1 : kBatches;      // unrolled, the wide forms outgrow the instruction cache
+  constexpr int kRow = kWidth < 2 * kBlockKeys ? 2 * kBlockKeys : kWidth;   // a warp's part also holds its weights
+  __shared__ __align__(16) float sm_o[kWarps][NQ][kRow];
+  __shared__ __align__(16) float sm_q[kWide ? NQ : 1][kWide ? kWidth : 4];
   __shared__ float sm_m[kWarps][NQ], sm_l[kWarps][NQ];
   __shared__ float cta_m[NQ], cta_l[NQ];
 
@@ -96,20 +126,31 @@ attention_direct_kernel(DirectArgs a) {
   const float* kh = a.k + head * a.nk * a.d;
   const float* vh = a.v + head * a.nk * a.dv;
 
-  float4 q[NQ];
-#pragma unroll
-  for (int i = 0; i < NQ; ++i)
-    q[i] = q0 + i < a.nq ? load_chunk(a.q + (head * a.nq + q0 + i) * a.d, sub * 4, a.d, a.vec)
+  float4 q[kWide ? 1 : NQ];
+  auto query = [&](int i, int chunk) {
+    return q0 + i < a.nq ? load_chunk(a.q + (head * a.nq + q0 + i) * a.d, chunk * 4, a.d, a.vec)
                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  };
+  if constexpr (kWide) {
+    for (int e = threadIdx.x; e < NQ * LP; e += kThreads)
+      *reinterpret_cast<float4*>(&sm_q[e / LP][e % LP * 4]) = query(e / LP, e % LP);
+    __syncthreads();
+  } else {
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) q[i] = query(i, sub);
+  }
+  // This warp's weights: its own part of sm_o, which is written after its last block of keys.
+  float2(*sm_p)[NQ] = reinterpret_cast<float2(*)[NQ]>(sm_o[warp]);
+  static_assert(sizeof(float2) * kBlockKeys * NQ <= sizeof(sm_o[0]), "the weights fit the warp's part");
   const float scale = a.logit_scale ? __ldg(a.logit_scale) : 1.0f;
 
   float m[NQ], l[NQ];
-  float4 o[NQ];
+  pair_t o[NQ][2];
 #pragma unroll
   for (int i = 0; i < NQ; ++i) {
     m[i] = -CUDART_INF_F;
     l[i] = 0.0f;
-    o[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    o[i][0] = o[i][1] = 0;
   }
 
   const size_t n_blocks = (a.nk + kBlockKeys - 1) / kBlockKeys;
@@ -118,7 +159,7 @@ attention_direct_kernel(DirectArgs a) {
   for (size_t blk = b_lo + warp; blk < b_hi; blk += kWarps) {
     const size_t key0 = blk * kBlockKeys;
     float s[NQ];
-#pragma unroll
+#pragma unroll kBatchUnroll
     for (int b = 0; b < kBatches; ++b) {
       float4 x[8];
 #pragma unroll
@@ -130,9 +171,13 @@ attention_direct_kernel(DirectArgs a) {
 #pragma unroll
       for (int i = 0; i < NQ; ++i) {
         float part[8];
+        const float4 qi = kWide ? *reinterpret_cast<const float4*>(&sm_q[kWide ? i : 0][kWide ? sub * 4 : 0]) : q[kWide ? 0 : i];
+        const pair_t q_lo = pack(qi.x, qi.y), q_hi = pack(qi.z, qi.w);
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          part[u] = fmaf(q[i].w, x[u].w, fmaf(q[i].z, x[u].z, fmaf(q[i].y, x[u].y, q[i].x * x[u].x)));
+        for (int u = 0; u < 8; ++u) {
+          const float2 t = unpack(fma2(q_hi, pack(x[u].z, x[u].w), mul2(q_lo, pack(x[u].x, x[u].y))));
+          part[u] = t.x + t.y;
+        }
         const float sum = sum_eight<LP>(part, sub);
         if (b == 0 || sub % kBatches == b) s[i] = sum;
       }
@@ -147,13 +192,22 @@ attention_direct_kernel(DirectArgs a) {
       if (top != m[i]) {                       // uniform: every lane holds the same two values
         const float shrink = weight_of(m[i], top);
         l[i] *= shrink;
-        o[i].x *= shrink; o[i].y *= shrink; o[i].z *= shrink; o[i].w *= shrink;
+        o[i][0] = mul2(o[i][0], pack(shrink, shrink));
+        o[i][1] = mul2(o[i][1], pack(shrink, shrink));
         m[i] = top;
       }
       s[i] = key < a.nk ? weight_of(s[i], top) : 0.0f;
       l[i] += s[i];
     }
+    if constexpr (kWide) {
+      __syncwarp();                            // the lanes have read the weights of the block before
+      const int slot = ((sub % kBatches) * 8 + sub / kBatches) * kKeysPerLoad + grp;
 #pragma unroll
+      for (int i = 0; i < NQ; i += 2)
+        *reinterpret_cast<float4*>(&sm_p[slot][i]) = make_float4(s[i], s[i], s[i + 1], s[i + 1]);
+      __syncwarp();
+    }
+#pragma unroll kBatchUnroll
     for (int b = 0; b < kBatches; ++b) {
       float4 x[8];
 #pragma unroll
@@ -164,31 +218,45 @@ attention_direct_kernel(DirectArgs a) {
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const int holder = grp * LP + u * kBatches + b;
+        const pair_t x_lo = pack(x[u].x, x[u].y), x_hi = pack(x[u].z, x[u].w);
+        if constexpr (kWide) {
+          const int slot = (b * 8 + u) * kKeysPerLoad + grp;
 #pragma unroll
-        for (int i = 0; i < NQ; ++i) {
-          const float p = __shfl_sync(0xffffffffu, s[i], holder);
-          o[i].x = fmaf(p, x[u].x, o[i].x);
-          o[i].y = fmaf(p, x[u].y, o[i].y);
-          o[i].z = fmaf(p, x[u].z, o[i].z);
-          o[i].w = fmaf(p, x[u].w, o[i].w);
+          for (int i = 0; i < NQ; i += 2) {
+            const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(&sm_p[slot][i]);
+            o[i][0] = fma2(p.x, x_lo, o[i][0]);
+            o[i][1] = fma2(p.x, x_hi, o[i][1]);
+            o[i + 1][0] = fma2(p.y, x_lo, o[i + 1][0]);
+            o[i + 1][1] = fma2(p.y, x_hi, o[i + 1][1]);
+          }
+        } else {
+          const int holder = grp * LP + u * kBatches + b;
+#pragma unroll
+          for (int i = 0; i < NQ; ++i) {
+            const float w = __shfl_sync(0xffffffffu, s[i], holder);
+            o[i][0] = fma2(pack(w, w), x_lo, o[i][0]);
+            o[i][1] = fma2(pack(w, w), x_hi, o[i][1]);
+          }
         }
       }
     }
   }
 
   // The warps of the CTA meet.
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < NQ; ++i) {
     l[i] = warp_fold<IB_OP_ADD>(l[i]);
+    const float2 lo = unpack(o[i][0]), hi = unpack(o[i][1]);
+    float4 sum = make_float4(lo.x, lo.y, hi.x, hi.y);
 #pragma unroll
     for (int off = LP; off < 32; off <<= 1) {
-      o[i].x += __shfl_xor_sync(0xffffffffu, o[i].x, off);
-      o[i].y += __shfl_xor_sync(0xffffffffu, o[i].y, off);
-      o[i].z += __shfl_xor_sync(0xffffffffu, o[i].z, off);
-      o[i].w += __shfl_xor_sync(0xffffffffu, o[i].w, off);
+      sum.x += __shfl_xor_sync(0xffffffffu, sum.x, off);
+      sum.y += __shfl_xor_sync(0xffffffffu, sum.y, off);
+      sum.z += __shfl_xor_sync(0xffffffffu, sum.z, off);
+      sum.w += __shfl_xor_sync(0xffffffffu, sum.w, off);
     }
-    if (grp == 0) *reinterpret_cast<float4*>(&sm_o[warp][i][sub * 4]) = o[i];
+    if (grp == 0) *reinterpret_cast<float4*>(&sm_o[warp][i][sub * 4]) = sum;
     if (lane == 0) {
       sm_m[warp][i] = m[i];
       sm_l[warp][i] = l[i];
@@ -243,27 +311,45 @@ attention_direct_kernel(DirectArgs a) {
   cluster.sync();                            // nobody leaves while its shared memory is read
 }
 
-// One warp per query row: merges the row's key ranges.
-__global__ void __launch_bounds__(kThreads)
+// One CTA per query row: merges the row's key ranges.  The ranges' weights are computed once, then
+// groups of 128 threads (one per column) each add a share of the ranges and meet in shared memory.
+constexpr int kMergeThreads = 512, kMergeGroups = kMergeThreads / 128, kMaxSplits = 512;
+
+__global__ void __launch_bounds__(kMergeThreads)
 attention_direct_merge_kernel(const float* __restrict__ partial_o, const float2* __restrict__ partial_ml,
-                              float* __restrict__ o, size_t rows, int splits, int dv) {
-  const int lane = threadIdx.x & 31;
-  const size_t row = static_cast<size_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const float2* ml = partial_ml + row * splits;
-  float top = -CUDART_INF_F;
-  for (int s = lane; s < splits; s += 32) top = fmaxf(top, ml[s].x);
-  top = warp_fold<IB_OP_MAX>(top);
-  float sum = 0.0f;
-  for (int s = lane; s < splits; s += 32) sum = fmaf(ml[s].y, weight_of(ml[s].x, top), sum);
-  sum = warp_fold<IB_OP_ADD>(sum);
-  for (int c = lane; c < dv; c += 32) {
-    float acc = 0.0f;
+                              float* __restrict__ o, int splits, int dv) {
+  __shared__ float weight[kMaxSplits], scratch[kMergeThreads / 32][2], meet[kMergeGroups][128];
+  const size_t row = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool mine = static_cast<int>(threadIdx.x) < splits;               // at most one range per thread
+  const float2 ml = mine ? partial_ml[row * splits + threadIdx.x] : make_float2(-CUDART_INF_F, 0.0f);
+  float top = warp_fold<IB_OP_MAX>(ml.x);
+  if (lane == 0) scratch[warp][0] = top;
+  __syncthreads();
+  top = scratch[0][0];
+#pragma unroll
+  for (int w = 1; w < kMergeThreads / 32; ++w) top = fmaxf(top, scratch[w][0]);
+  const float f = mine ? weight_of(ml.x, top) : 0.0f;
+  if (mine) weight[threadIdx.x] = f;
+  const float part = warp_fold<IB_OP_ADD>(ml.y * f);
+  if (lane == 0) scratch[warp][1] = part;
+  __syncthreads();
+  const int c = threadIdx.x % 128, group = threadIdx.x / 128;
+  float acc = 0.0f;
+  if (c < dv) {
+    const float* at = partial_o + row * splits * dv + c;
 #pragma unroll 8
-    for (int s = 0; s < splits; ++s)
-      acc = fmaf(partial_o[(row * splits + s) * dv + c], weight_of(ml[s].x, top), acc);
-    o[row * dv + c] = acc / sum;
+    for (int s = group; s < splits; s += kMergeGroups) acc = fmaf(at[static_cast<size_t>(s) * dv], weight[s], acc);
   }
+  meet[group][c] = acc;
+  __syncthreads();
+  if (group != 0 || c >= dv) return;
+  float sum = 0.0f;
+#pragma unroll
+  for (int w = 0; w < kMergeThreads / 32; ++w) sum += scratch[w][1];
+#pragma unroll
+  for (int g = 1; g < kMergeGroups; ++g) acc += meet[g][c];
+  o[row * dv + c] = acc / sum;
 }
 
 struct DirectPlan {
@@ -288,7 +374,7 @@ DirectPlan direct_plan(size_t batch, size_t nq, size_t nk) {
   const size_t room = static_cast<size_t>(kNumSMs) * (n >= 4 ? 2 : 3);
   size_t splits = units ? room / units : 1;
   if (splits > blocks / kWarps) splits = blocks / kWarps;
-  if (splits > 512) splits = 512;
+  if (splits > static_cast<size_t>(kMaxSplits)) splits = kMaxSplits;
   if (splits > static_cast<size_t>(kMaxCluster) && splits < 2 * static_cast<size_t>(kMaxCluster)) splits = kMaxCluster;
   if (splits < 1) splits = 1;
   const size_t per = (blocks + splits - 1) / splits;
@@ -370,9 +456,8 @@ int attention_direct(const float* q, const float* k, const float* v, float* o, s
   }
   count_launch();
   if (p.splits == 1 || p.cluster) return 0;
-  const size_t rows = batch * nq;
-  attention_direct_merge_kernel<<<static_cast<unsigned>((rows + kWarps - 1) / kWarps), kThreads, 0, s>>>(
-      a.partial_o, a.partial_ml, o, rows, p.splits, a.dv);
+  attention_direct_merge_kernel<<<static_cast<unsigned>(batch * nq), kMergeThreads, 0, s>>>(
+      a.partial_o, a.partial_ml, o, p.splits, a.dv);
   return check_launch("ib_attention (fp32 merge)");
 }
 
