@@ -30,7 +30,8 @@ SOURCES = [
     "kernels/map.cu",
     "kernels/reduce.cu",
     "kernels/softmax.cu",
-    "kernels/contract_simt.cu",
+    "kernels/prepare_operands.cu",
+    "kernels/contract_fp32.cu",
     "kernels/device_util.cu",
     "kernels/gemm_tcgen05.cu",
     "kernels/attention_tcgen05.cu",

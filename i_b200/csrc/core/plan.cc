@@ -704,8 +704,7 @@ std::string Plan::describe() const {
            << (s.form.b_kmajor ? "[n,k]" : "[k,n]") << (s.form.swap_out ? ", output [n,m]" : "")
            << "\n";
         if (!s.chain.empty()) {
-          os << "    epilogue (applied to each element before it is stored; a separate pass on the "
-                "fp32 arm):";
+          os << "    epilogue (applied to each element before it is stored):";
           auto name = [&](int code) -> std::string {
             if (code == kChainPrev) return "_";
             return buffer_name(s.epilogue_in[code].buffer);

@@ -1,0 +1,362 @@
+// CUDA-core fp32 contraction: the IB_PRECISION_FP32 arm of ib_contract, and what AUTO takes for
+// products too small or too ragged for the tensor path (odd K, tiny tiles such as the 8x16x7 product
+// of ilang-python/test.py:52-56).  C[b][i][j] = sum_k A(b,i,k) B(b,j,k), the arithmetic of the
+// reference's loop nest (ilang-python/annotated-flashattn.c:57-89) up to summation order and FMA
+// contraction.
+//
+// Bound: the FMA pipes, 128 multiply-adds per clock and SM.  What keeps a tile kernel from them is
+// issue slots and shared-memory reads, so a thread owns TM x TN results (8 x 8 in the large tiles),
+// reads both operands as 16-byte quads (4 reads for 64 multiply-adds) and multiplies with fma.rn.f32x2,
+// two results per instruction (32 instead of 64 a step, each lane rounded as a plain fma).  Tiles of
+// both operands go through registers into [k][row] shared memory whatever their layout, the next
+// tile's loads in flight while the current one is multiplied, one barrier per tile.
+//
+// Results too few for the machine: a product is cut along k into up to eight parts, the CTAs of one
+// cluster, whose sums meet in distributed shared memory: no workspace, no second launch, a fixed
+// order.  Tile and parts are chosen by an estimate (choose below).
+//
+// Measured on B200, against 64 x 64 tiles of 4 x 4 results with 4-byte shared-memory reads: 1024 x
+// 1000 x 1001 145 -> 62 us, 2048 x 2048 x 512 105 us (41 TFLOP/s; the FMA pipe is 66-69 % busy, held
+// by the waits between a quad's packing and its use), 32 x 32 x 2048 226 -> 10 us.
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace ib {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kMaxParts = 8;               // portable cluster size
+
+struct Operand {
+  const float* p;
+  size_t rows;                             // m or n
+  bool vec;                                // 16-byte loads along its contiguous axis
+};
+
+struct Fp32Args {
+  Operand a, b;
+  float* c;
+  size_t k, k_len;
+  unsigned tiles_n, parts;
+  bool c_vec;
+};
+
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long both(float x) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 halves(unsigned long long x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+
+// A thread's share of an operand's ROWS x 16 tile on its way to shared memory.
+template <int ROWS, int TK, int THREADS, bool KMAJOR>
+struct Stage {
+  static constexpr int kPer = ROWS * TK / THREADS;
+  static_assert(kPer % 4 == 0, "whole quads per thread");
+  float v[kPer];
+
+  __device__ __forceinline__ void load(const Operand& op, const float* base, size_t row0, size_t k, size_t k0,
+                                       size_t k_hi) {
+    if (op.vec) {
+#pragma unroll
+      for (int i = 0; i < kPer / 4; ++i) {
+        const int e = threadIdx.x + i * THREADS;
+        const int row = KMAJOR ? e / (TK / 4) : (e % (ROWS / 4)) * 4, kk = KMAJOR ? (e % (TK / 4)) * 4 : e / (ROWS / 4);
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (row0 + row < op.rows && k0 + kk < k_hi)
+          x = __ldg(reinterpret_cast<const float4*>(KMAJOR ? base + (row0 + row) * k + k0 + kk
+                                                           : base + (k0 + kk) * op.rows + row0 + row));
+        v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int e = threadIdx.x + i * THREADS;
+        const int row = KMAJOR ? e / TK : e % ROWS, kk = KMAJOR ? e % TK : e / ROWS;
+        v[i] = row0 + row < op.rows && k0 + kk < k_hi
+                   ? __ldg(KMAJOR ? base + (row0 + row) * k + k0 + kk : base + (k0 + kk) * op.rows + row0 + row)
+                   : 0.0f;
+      }
+    }
+  }
+
+  __device__ __forceinline__ void store(float (*tile)[ROWS + 4], bool vec) const {
+    if (vec) {
+#pragma unroll
+      for (int i = 0; i < kPer / 4; ++i) {
+        const int e = threadIdx.x + i * THREADS;
+        if (KMAJOR) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tile[(e % (TK / 4)) * 4 + j][e / (TK / 4)] = v[4 * i + j];
+        } else {
+          *reinterpret_cast<float4*>(&tile[e / (ROWS / 4)][(e % (ROWS / 4)) * 4]) =
+              make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int e = threadIdx.x + i * THREADS;
+        tile[KMAJOR ? e % TK : e / ROWS][KMAJOR ? e / TK : e % ROWS] = v[i];
+      }
+    }
+  }
+};
+
+// The caller's pointwise operators on four neighbouring results of one row; the arithmetic of the
+// pointwise kernels (a call of its own, so nothing is contracted across operators).
+__device__ __noinline__ float4 fp32_epilogue(const GemmEpilogue& e, float4 r, size_t grow, size_t col, size_t n) {
+  float v[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll 1
+  for (int k = 0; k < e.n_ops; ++k) {
+    const int w = e.which[k];
+    float t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      t[j] = 0.0f;
+      if (w >= 0 && col + j < n) {
+        const float* p = e.operand[w];
+        const int mode = e.mode[w];
+        t[j] = __ldg(mode == 0 ? p + grow * n + col + j : mode == 1 ? p + grow : mode == 2 ? p + col + j : p);
+      }
+    }
+    const bool right = e.acc_right[k] != 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[j] = w < 0 ? apply_unary(e.op[k], v[j]) : right ? apply_binary(e.op[k], t[j], v[j]) : apply_binary(e.op[k], v[j], t[j]);
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+__device__ __forceinline__ void put_quad(float* c, float4 r, size_t grow, size_t col, size_t n, bool vec,
+                                         const GemmEpilogue& e) {
+  if (e.n_ops) r = fp32_epilogue(e, r, grow, col, n);
+  float* at = c + grow * n + col;
+  if (vec && col + 4 <= n) {
+    *reinterpret_cast<float4*>(at) = r;
+  } else {
+    if (col < n) at[0] = r.x;
+    if (col + 1 < n) at[1] = r.y;
+    if (col + 2 < n) at[2] = r.z;
+    if (col + 3 < n) at[3] = r.w;
+  }
+}
+
+template <int BM, int BN, int TK, int TM, int TN, bool AK, bool BK>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), 512 / ((BM / TM) * (BN / TN)))
+contract_fp32_kernel(const __grid_constant__ Fp32Args g, const __grid_constant__ GemmEpilogue epilogue) {
+  constexpr int kThreads = (BM / TM) * (BN / TN);
+  constexpr int kQm = TM / 4, kQn = TN / 4;
+  constexpr int kAcross = BN / TN;           // threads along a row of results
+  constexpr size_t kTileFloats = 2 * TK * (BM + 4 + BN + 4);
+  constexpr size_t kMeetFloats = BM * BN <= 64 * 128 ? BM * BN : 0;      // larger tiles are never cut along k
+  __shared__ __align__(16) float smem[kTileFloats > kMeetFloats ? kTileFloats : kMeetFloats];
+  float(*sa)[TK][BM + 4] = reinterpret_cast<float(*)[TK][BM + 4]>(smem);
+  float(*sb)[TK][BN + 4] = reinterpret_cast<float(*)[TK][BN + 4]>(smem + 2 * TK * (BM + 4));
+
+  const unsigned tile = blockIdx.x / g.parts, part = blockIdx.x - tile * g.parts;
+  const size_t i0 = static_cast<size_t>(tile / g.tiles_n) * BM, j0 = static_cast<size_t>(tile % g.tiles_n) * BN;
+  const size_t m = g.a.rows, n = g.b.rows, batch = blockIdx.y;
+  const float* a = g.a.p + batch * m * g.k;
+  const float* b = g.b.p + batch * n * g.k;
+  const size_t k_lo = part * g.k_len, k_hi = k_lo + g.k_len < g.k ? k_lo + g.k_len : g.k;
+  const int tx = threadIdx.x % kAcross, ty = threadIdx.x / kAcross;
+
+  unsigned long long acc[TM][TN / 2];
+#pragma unroll
+  for (int u = 0; u < TM; ++u)
+#pragma unroll
+    for (int w = 0; w < TN / 2; ++w) acc[u][w] = 0;
+
+  Stage<BM, TK, kThreads, AK> fa;
+  Stage<BN, TK, kThreads, BK> fb;
+  if (k_lo < k_hi) {
+    fa.load(g.a, a, i0, g.k, k_lo, k_hi);
+    fb.load(g.b, b, j0, g.k, k_lo, k_hi);
+    fa.store(sa[0], g.a.vec);
+    fb.store(sb[0], g.b.vec);
+  }
+  __syncthreads();
+  int buf = 0;
+  for (size_t k0 = k_lo; k0 < k_hi; k0 += TK) {
+    const bool more = k0 + TK < k_hi;
+    if (more) {
+      fa.load(g.a, a, i0, g.k, k0 + TK, k_hi);
+      fb.load(g.b, b, j0, g.k, k0 + TK, k_hi);
+    }
+#pragma unroll
+    for (int kk = 0; kk < TK; ++kk) {
+      float av[TM];
+      unsigned long long bv[TN / 2];
+#pragma unroll
+      for (int q = 0; q < kQm; ++q)
+        *reinterpret_cast<float4*>(&av[4 * q]) = *reinterpret_cast<const float4*>(&sa[buf][kk][q * (BM / kQm) + ty * 4]);
+#pragma unroll
+      for (int q = 0; q < kQn; ++q)
+        *reinterpret_cast<ulonglong2*>(&bv[2 * q]) =
+            *reinterpret_cast<const ulonglong2*>(&sb[buf][kk][q * (BN / kQn) + tx * 4]);
+#pragma unroll
+      for (int u = 0; u < TM; ++u) {
+        const unsigned long long aa = both(av[u]);
+#pragma unroll
+        for (int w = 0; w < TN / 2; ++w) fma2(acc[u][w], aa, bv[w]);
+      }
+    }
+    if (more) {
+      fa.store(sa[buf ^ 1], g.a.vec);
+      fb.store(sb[buf ^ 1], g.b.vec);
+    }
+    __syncthreads();
+    buf ^= 1;
+  }
+
+  if (g.parts == 1) {
+#pragma unroll
+    for (int u = 0; u < TM; ++u) {
+      const size_t gi = i0 + (u / 4) * (BM / kQm) + ty * 4 + u % 4;
+      if (gi >= m) continue;
+#pragma unroll
+      for (int q = 0; q < kQn; ++q) {
+        const float2 lo = halves(acc[u][2 * q]), hi = halves(acc[u][2 * q + 1]);
+        put_quad(g.c, make_float4(lo.x, lo.y, hi.x, hi.y), batch * m + gi, j0 + q * (BN / kQn) + tx * 4, n, g.c_vec,
+                 epilogue);
+      }
+    }
+    return;
+  }
+  if constexpr (kMeetFloats > 0) {
+    // The parts meet: every CTA leaves its sums in shared memory, each adds a share of the tile.
+    float4* meet = reinterpret_cast<float4*>(smem);
+#pragma unroll
+    for (int u = 0; u < TM; ++u)
+#pragma unroll
+      for (int q = 0; q < kQn; ++q) {
+        const float2 lo = halves(acc[u][2 * q]), hi = halves(acc[u][2 * q + 1]);
+        meet[((u / 4) * (BM / kQm) + ty * 4 + u % 4) * (BN / 4) + q * (BN / kQn) / 4 + tx] =
+            make_float4(lo.x, lo.y, hi.x, hi.y);
+      }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    for (unsigned e = part * kThreads + threadIdx.x; e < BM * BN / 4; e += g.parts * kThreads) {
+      const size_t gi = i0 + e / (BN / 4), gj = j0 + (e % (BN / 4)) * 4;
+      if (gi >= m || gj >= n) continue;
+      float4 x[kMaxParts];
+#pragma unroll
+      for (unsigned p = 0; p < kMaxParts; ++p)
+        if (p < g.parts) x[p] = *cluster.map_shared_rank(&meet[e], p);
+      float4 sum = x[0];
+#pragma unroll
+      for (unsigned p = 1; p < kMaxParts; ++p)
+        if (p < g.parts) {
+          sum.x += x[p].x; sum.y += x[p].y; sum.z += x[p].z; sum.w += x[p].w;
+        }
+      put_quad(g.c, sum, batch * m + gi, gj, n, g.c_vec, epilogue);
+    }
+    cluster.sync();                          // nobody leaves while its shared memory is read
+  }
+}
+
+struct Choice {
+  int tile;                                  // index into the tile list
+  size_t parts;
+};
+
+struct TileShape {
+  size_t bm, bn;
+  double one, most;                          // share of the FMA rate with one CTA on an SM, with several
+};
+constexpr TileShape kTiles[] = {{128, 128, 0.53, 0.68}, {64, 128, 0.45, 0.65}, {64, 64, 0.30, 0.55}, {32, 32, 0.13, 0.34}};
+
+// Tile and parts with the least estimated time: the busiest SM's share of the multiply-adds at the
+// rate its number of resident CTAs reaches, plus a cost for the meeting of parts.  The rates are
+// measured (one CTA: latency of shared memory and loads is exposed; several: it is covered), as is the
+// meeting (about 1.5 us more for a cluster launch and its two barriers).
+Choice choose(size_t batch, size_t m, size_t n, size_t k) {
+  Choice best{3, 1};
+  double best_time = 1e300;
+  for (int t = 0; t < 4; ++t) {
+    const TileShape& s = kTiles[t];
+    const double tiles = static_cast<double>(batch) * ((m + s.bm - 1) / s.bm) * ((n + s.bn - 1) / s.bn);
+    for (size_t parts = 1; parts <= static_cast<size_t>(kMaxParts); ++parts) {
+      if (parts > 1 && (t == 0 || k < parts * 2 * 16)) break;
+      const double per_sm = static_cast<double>(static_cast<size_t>((tiles * parts + kNumSMs - 1) / kNumSMs));
+      const size_t k_len = ((k + parts - 1) / parts + 16 - 1) / 16 * 16;
+      const double rate = s.one * per_sm < s.most ? s.one * per_sm : s.most;
+      const double time = per_sm * k_len * s.bm * s.bn / 128 / rate + (parts > 1 ? 3000 + 0.15 * s.bm * s.bn / 4 : 0);
+      if (time < best_time) {
+        best_time = time;
+        best = Choice{t, parts};
+      }
+    }
+  }
+  return best;
+}
+
+template <int BM, int BN, int TK, int TM, int TN>
+cudaError_t launch_tile(Fp32Args g, const GemmEpilogue& e, size_t batch, size_t parts, bool ak, bool bk,
+                        cudaStream_t s) {
+  const size_t tiles_m = (g.a.rows + BM - 1) / BM, tiles_n = (g.b.rows + BN - 1) / BN;
+  const size_t ctas = tiles_m * tiles_n * parts;
+  if (ctas > 0x7fffffffu || tiles_n > 0x7fffffffu) return cudaErrorInvalidConfiguration;
+  g.tiles_n = static_cast<unsigned>(tiles_n);
+  g.parts = static_cast<unsigned>(parts);
+  // Whole k-tiles per part, so that every part but the last is full.
+  g.k_len = ((g.k + parts - 1) / parts + TK - 1) / TK * TK;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(parts);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), static_cast<unsigned>(batch));
+  cfg.blockDim = dim3((BM / TM) * (BN / TN));
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = parts > 1 ? 1 : 0;
+  if (ak) return bk ? cudaLaunchKernelEx(&cfg, contract_fp32_kernel<BM, BN, TK, TM, TN, true, true>, g, e)
+                    : cudaLaunchKernelEx(&cfg, contract_fp32_kernel<BM, BN, TK, TM, TN, true, false>, g, e);
+  return bk ? cudaLaunchKernelEx(&cfg, contract_fp32_kernel<BM, BN, TK, TM, TN, false, true>, g, e)
+            : cudaLaunchKernelEx(&cfg, contract_fp32_kernel<BM, BN, TK, TM, TN, false, false>, g, e);
+}
+
+}  // namespace
+
+int contract_fp32(const float* a, const float* b, float* c, size_t batch, size_t m, size_t n, size_t k,
+                  bool a_kmajor, bool b_kmajor, cudaStream_t s, const GemmEpilogue* e) {
+  if (batch == 0 || m == 0 || n == 0) return 0;
+  if (batch > 65535) return fail("ib_contract: more than 65535 batch entries");
+  // 16-byte loads need every row of the operand, in every batch entry, to start on 16 bytes.
+  Fp32Args g{};
+  g.a = Operand{a, m, (a_kmajor ? k : m) % 4 == 0 && aligned16(a)};
+  g.b = Operand{b, n, (b_kmajor ? k : n) % 4 == 0 && aligned16(b)};
+  g.c = c;
+  g.k = k;
+  g.c_vec = n % 4 == 0 && aligned16(c);
+  const Choice pick = choose(batch, m, n, k);
+  const GemmEpilogue none{};
+  const GemmEpilogue& ep = e ? *e : none;
+  cudaError_t err;
+  switch (pick.tile) {
+    case 0: err = launch_tile<128, 128, 16, 8, 8>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
+    case 1: err = launch_tile<64, 128, 16, 8, 8>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
+    case 2: err = launch_tile<64, 64, 32, 8, 4>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
+    default: err = launch_tile<32, 32, 32, 4, 4>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
+  }
+  if (err != cudaSuccess) {
+    cudaGetLastError();
+    return fail(std::string("ib_contract (fp32): ") + cudaGetErrorString(err));
+  }
+  count_launch();
+  return 0;
+}
+
+}  // namespace ib

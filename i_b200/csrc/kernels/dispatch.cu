@@ -41,25 +41,18 @@ size_t carve_bytes(size_t floats) {
   return floats > kMaxFloats ? SIZE_MAX >> 4 : round_up(floats * sizeof(float), 256);
 }
 
-// Parts into which the k range of a contraction with few output tiles is cut, so that every SM
-// has work: an output of 128 x 128 is four tiles of the fp32 arm (one of the tensor arm), and a
-// k of thousands would run on that many SMs.  Each part sums into its own copy of the result
-// and the copies are added.  `tile`: output rows and columns per CTA of the arm.  1 = whole.
-size_t k_parts(size_t batch, size_t m, size_t n, size_t k, size_t tile) {
-  const size_t tiles = batch * ((m + tile - 1) / tile) * ((n + tile - 1) / tile);
-  if (tiles == 0 || tiles * 2 > static_cast<size_t>(kNumSMs) || k < 1024) return 1;
+// Parts into which the TF32 tensor arm cuts the k range of a contraction with few output tiles, so
+// that every SM has work: an output of 128 x 128 is one tile, and a k of thousands would run on one
+// SM.  Each part sums into its own copy of the result and the copies are added.  The parts are batch
+// entries of one tensor map: one batch entry only, and parts of equal length, a multiple of four.
+// 1 = whole.  (The fp32 arm cuts its k range inside a cluster.)
+size_t k_parts_tensor(size_t batch, size_t m, size_t n, size_t k) {
+  const size_t tiles = ((m + 127) / 128) * ((n + 127) / 128);
+  if (batch != 1 || tiles == 0 || tiles * 2 > static_cast<size_t>(kNumSMs) || k < 1024) return 1;
   size_t parts = static_cast<size_t>(kNumSMs) * 2 / tiles;
   if (parts > k / 128) parts = k / 128;
   if (parts > 64) parts = 64;
-  if (batch * parts > 65535) parts = 65535 / batch;
-  return parts < 2 ? 1 : parts;
-}
-
-// The same for the TF32 tensor arm, which takes the parts as batch entries of one tensor map:
-// one batch entry only, and parts of equal length, a multiple of four.
-size_t k_parts_tensor(size_t batch, size_t m, size_t n, size_t k) {
-  if (batch != 1) return 1;
-  for (size_t parts = k_parts(1, m, n, k, 128); parts >= 2; --parts)
+  for (; parts >= 2; --parts)
     if (k % (4 * parts) == 0) return parts;
   return 1;
 }
@@ -88,11 +81,13 @@ bool attention_shape_ok(size_t d, size_t dv) {
 // Attention straight from K and V in fp32 (attention_direct.cu).  Two rules:
 //   up to kDirectQueries queries per head, under every precision: the pass is then bound by reading K
 //   and V once, which the tensor arms cannot do (they first write converted copies of both, as many
-//   bytes again), and no arm is less exact;
-//   otherwise fp32 arithmetic up to kDirectFlop: above that two tiled contractions with the scores in
-//   memory between them are faster.
+//   bytes again), and no arm is less exact.  32 heads x 10000 keys x 128 on B200, direct / fp16 arm /
+//   bf16 arm: 4 queries 80 / 207 / 135 us, 8 queries 115 / 207 / 136, 16 queries 204 / 210 / 139;
+//   otherwise fp32 arithmetic up to kDirectFlop: above, two tiled contractions with the scores in
+//   memory between them are faster (8 x 256 x 256 x 64, 2^27: 17.6 / 19.7 us; 1024 x 1024 x 64, 2^28:
+//   30.6 / 26.8).
 constexpr size_t kDirectQueries = 8;
-constexpr double kDirectFlop = 1073741824.0;    // 2^30
+constexpr double kDirectFlop = 134217728.0;     // 2^27
 bool attention_prefers_direct(size_t batch, size_t nq, size_t nk, size_t d, size_t dv, bool v_kmajor, int precision) {
   if (v_kmajor || !attention_direct_shape_ok(batch, nq, nk, d, dv)) return false;
   if (nq <= kDirectQueries) return true;
@@ -234,10 +229,7 @@ extern "C" size_t ib_contract_workspace_bytes(size_t batch, size_t m, size_t n, 
     return carve_bytes(long_rows_floats(batch, k));   // dot products of few, very long rows
   }
   const double flop = 2.0 * batch * m * n * k;
-  // Copies of the result when the k range is cut into parts (either 32-bit arm).
-  const size_t parts = std::max(k_parts(batch, m, n, k, 64), k_parts_tensor(batch, m, n, k));
-  const size_t copies = parts > 1 ? carve_bytes(batch * parts * m * n) : 0;
-  if (!wants_tensor(precision, flop)) return copies;
+  if (!wants_tensor(precision, flop)) return 0;
   if (precision == IB_PRECISION_AUTO && contract_prefers_f16(m, n, k)) precision = IB_PRECISION_F16;
   if (precision == IB_PRECISION_F16) {
     // fp16 copies of both operands plus one scale per row; fp32 transposes first when needed.
@@ -256,8 +248,10 @@ extern "C" size_t ib_contract_workspace_bytes(size_t batch, size_t m, size_t n, 
     if (!b_kmajor) bytes += carve_bytes(batch * n * k);
     return bytes;
   }
-  if (!contract_shape_ok(k)) return copies;
-  size_t bytes = copies;
+  if (!contract_shape_ok(k)) return 0;
+  // Copies of the result when the k range is cut into parts.
+  const size_t parts = k_parts_tensor(batch, m, n, k);
+  size_t bytes = parts > 1 ? carve_bytes(batch * parts * m * n) : 0;
   if (!a_kmajor) bytes += carve_bytes(batch * m * k);
   if (!b_kmajor) bytes += carve_bytes(batch * n * k);
   return bytes;
@@ -291,9 +285,9 @@ extern "C" int ib_contract(const float* a, const float* b, float* c, size_t batc
 namespace ib {
 namespace {
 
-// Pointwise operators that follow a contraction, in the two forms its arms need: `fused` for the
-// tensor-core kernels' epilogue, and the same list as an ib_map_chain call over the stored result
-// for the arms that have no epilogue hook (fp32, and a contraction over no terms).
+// Pointwise operators that follow a contraction, in the two forms it needs: `fused` for the tile
+// kernels' epilogue, and the same list as an ib_map_chain call over the stored result for the routes
+// that have no epilogue hook (folds, parts added afterwards, and a contraction over no terms).
 struct ContractChain {
   GemmEpilogue fused;
   int n_ops = 0;
@@ -386,18 +380,6 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
   const GemmEpilogue* fused = chain ? &chain->fused : nullptr;
   auto then_chain = [&](int rc) {
     return rc != 0 || !chain ? rc : chain->in_place(c, batch * m, n, stream);
-  };
-  // The fp32 arm, its k range in parts when the output has too few tiles for the machine and the
-  // workspace has room for the copies.
-  auto simt = [&](const float* pa, const float* pb, bool a_km, bool b_km, Carver& ws) {
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t parts = k_parts(batch, m, n, k, 64);
-    float* copies = parts > 1 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0
-                        ? ws.take(batch * parts * m * n)
-                        : nullptr;
-    if (!copies) return contract_simt(pa, pb, c, batch, m, n, k, a_km, b_km, st);
-    if (int rc = contract_simt(pa, pb, copies, batch, m, n, k, a_km, b_km, st, parts)) return rc;
-    return sum_partials(copies, c, batch, parts, m * n, st);
   };
   if (col_tile != 0 && col_tile != 128 && col_tile != 256)
     return fail("ib_contract: col_tile must be 0, 128 or 256");
@@ -552,10 +534,9 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
       return then_chain(sum_partials(copies, c, 1, parts, m * n, s));
     }
     // Misaligned base pointers: the fp32 arm takes any layout.
-    return then_chain(simt(ak, bk, true, true, ws));
+    return contract_fp32(ak, bk, c, batch, m, n, k, true, true, s, fused);
   }
-  Carver ws(workspace, workspace_bytes);
-  return then_chain(simt(a, b, a_kmajor != 0, b_kmajor != 0, ws));
+  return contract_fp32(a, b, c, batch, m, n, k, a_kmajor != 0, b_kmajor != 0, s, fused);
 }
 
 }  // namespace

@@ -1,14 +1,7 @@
-// CUDA-core fp32 contraction and layout helpers.
+// Layout and type changes ahead of the tensor-core kernels.
 //
-// ib::contract_simt is the IB_PRECISION_FP32 arm of ib_contract: shared-memory
-// tiled FMA GEMM for problems that are too small or too ragged for the tensor
-// path (odd K, tiny tiles such as the 8x16x7 product of ilang-python/test.py:
-// 52-56).  It computes C[b][i][j] = sum_k A(b,i,k) B(b,j,k) in fp32, the same
-// arithmetic as the reference's loop nest (ilang-python/annotated-flashattn.c:
-// 57-89) up to summation order and FMA contraction.
-//
-// ib::transpose_batched rewrites [b][r][c] as [b][c][r]; the tensor path uses
-// it to give tcgen05 K-major operands.
+// ib::transpose_batched rewrites [b][r][c] as [b][c][r] (K-major operands for tcgen05, and the
+// `ij~ji` copies); the rest rounds or converts the operands of contractions and of fused attention.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -20,70 +13,6 @@
 
 namespace ib {
 namespace {
-
-constexpr int kTile = 64;
-constexpr int kTileK = 16;
-
-template <bool A_KMAJOR, bool B_KMAJOR>
-__global__ void __launch_bounds__(256)
-contract_simt_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                     float* __restrict__ c, size_t m, size_t n, size_t k, size_t splits, size_t k_len) {
-  __shared__ float sa[kTileK][kTile + 1];
-  __shared__ float sb[kTileK][kTile + 1];
-  // blockIdx.z = batch entry * splits + split: a split sums k_len terms of the contraction into
-  // its own copy of the result (the caller adds the copies).
-  const size_t batch = blockIdx.z / splits, split = blockIdx.z - batch * splits;
-  a += batch * m * k;
-  b += batch * n * k;
-  c += static_cast<size_t>(blockIdx.z) * m * n;
-  const size_t k_lo = split * k_len, k_hi = k_lo + k_len < k ? k_lo + k_len : k;
-  const size_t i0 = static_cast<size_t>(blockIdx.y) * kTile;
-  const size_t j0 = static_cast<size_t>(blockIdx.x) * kTile;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (size_t k0 = k_lo; k0 < k_hi; k0 += kTileK) {
-    for (int e = threadIdx.x; e < kTile * kTileK; e += 256) {
-      // Walk the operand along its contiguous axis.
-      int row, kk;
-      if (A_KMAJOR) { row = e / kTileK; kk = e % kTileK; } else { kk = e / kTile; row = e % kTile; }
-      size_t gi = i0 + row, gk = k0 + kk;
-      float v = 0.0f;
-      if (gi < m && gk < k_hi) v = A_KMAJOR ? a[gi * k + gk] : a[gk * m + gi];
-      sa[kk][row] = v;
-      if (B_KMAJOR) { row = e / kTileK; kk = e % kTileK; } else { kk = e / kTile; row = e % kTile; }
-      size_t gj = j0 + row;
-      gk = k0 + kk;
-      v = 0.0f;
-      if (gj < n && gk < k_hi) v = B_KMAJOR ? b[gj * k + gk] : b[gk * n + gj];
-      sb[kk][row] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kTileK; ++kk) {
-      float av[4], bv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        av[u] = sa[kk][ty * 4 + u];
-        bv[u] = sb[kk][tx * 4 + u];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int w = 0; w < 4; ++w) acc[u][w] = fmaf(av[u], bv[w], acc[u][w]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    size_t gi = i0 + ty * 4 + u;
-    if (gi >= m) continue;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      size_t gj = j0 + tx * 4 + w;
-      if (gj < n) c[gi * n + gj] = acc[u][w];
-    }
-  }
-}
 
 // Round-to-nearest fp32 -> tf32 (10-bit mantissa, low 13 bits cleared).  The
 // tensor core itself truncates; rounding operands first halves the error and
@@ -926,27 +855,6 @@ int round_tf32_rows(const float* in0, float* out0, size_t rows0, size_t cols0, s
   dim3 grid(static_cast<unsigned>(blocks), in1 ? 2 : 1);
   round_rows_kernel<<<grid, 256, 0, s>>>(j0, j1);
   return check_launch("round_tf32");
-}
-
-int contract_simt(const float* a, const float* b, float* c, size_t batch, size_t m, size_t n,
-                  size_t k, bool a_kmajor, bool b_kmajor, cudaStream_t s, size_t splits) {
-  if (batch == 0 || m == 0 || n == 0) return 0;
-  if (splits < 1) splits = 1;
-  if (batch * splits > 65535) return fail("ib_contract: more than 65535 batch entries");
-  // Whole k-tiles per split, so that every split but the last is full.
-  const size_t k_len = ((k + splits - 1) / splits + kTileK - 1) / kTileK * kTileK;
-  dim3 grid(static_cast<unsigned>((n + kTile - 1) / kTile),
-            static_cast<unsigned>((m + kTile - 1) / kTile), static_cast<unsigned>(batch * splits));
-  if (grid.y > 65535) return fail("ib_contract: row count too large for the fp32 arm");
-  if (a_kmajor && b_kmajor)
-    contract_simt_kernel<true, true><<<grid, 256, 0, s>>>(a, b, c, m, n, k, splits, k_len);
-  else if (a_kmajor && !b_kmajor)
-    contract_simt_kernel<true, false><<<grid, 256, 0, s>>>(a, b, c, m, n, k, splits, k_len);
-  else if (!a_kmajor && b_kmajor)
-    contract_simt_kernel<false, true><<<grid, 256, 0, s>>>(a, b, c, m, n, k, splits, k_len);
-  else
-    contract_simt_kernel<false, false><<<grid, 256, 0, s>>>(a, b, c, m, n, k, splits, k_len);
-  return check_launch("ib_contract (fp32)");
 }
 
 int transpose_batched(const float* in, float* out, size_t batch, size_t rows, size_t cols,

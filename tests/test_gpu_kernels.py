@@ -466,6 +466,21 @@ def run_contract(lib, torch, a, b, akm, bkm, precision, batch=None):
     return out[0] if batch is None else out
 
 
+@pytest.mark.parametrize("batch,m,n,k", [
+    (1, 33, 31, 31), (1, 32, 32, 2048), (3, 70, 50, 515),        # the smallest tile, whole and cut along k
+    (1, 8, 8000, 40), (8, 300, 300, 128),                        # the middle tiles
+    (1, 1000, 1030, 257), (1, 1920, 2049, 129)])                 # the large ones
+@pytest.mark.parametrize("akm,bkm", [(True, True), (True, False), (False, True), (False, False)])
+def test_contract_fp32_tiles_and_parts(lib, torch, batch, m, n, k, akm, bkm):
+    # Every tile of the fp32 arm, whole and in parts along k, all layouts, against float64: k products
+    # rounded once each and summed in fp32, 1e-5 of the peak as elsewhere on this arm.
+    a, b = rand((batch,) + ((m, k) if akm else (k, m)), 94), rand((batch,) + ((n, k) if bkm else (k, n)), 95)
+    got = run_contract(lib, torch, a, b, akm, bkm, FP32, batch=batch)
+    want = np.einsum("bik,bjk->bij" if akm and bkm else "bik,bkj->bij" if akm else "bki,bjk->bij" if bkm else "bki,bkj->bij",
+                     a.astype(np.float64), b.astype(np.float64), optimize=True)
+    assert max_rel_to_peak(np.asarray(got).reshape(want.shape), want) <= TOL_FP32
+
+
 @pytest.mark.parametrize("m,n,k,akm,bkm", [
     (8, 7, 16, True, False),      # ilang-python/test.py:40-59
     (100, 40, 33, True, True), (65, 130, 17, False, True), (64, 64, 64, False, False),
