@@ -30,6 +30,7 @@ SOURCES = [
     "kernels/map.cu",
     "kernels/reduce.cu",
     "kernels/softmax.cu",
+    "kernels/expsum.cu",
     "kernels/prepare_operands.cu",
     "kernels/contract_fp32.cu",
     "kernels/device_util.cu",

@@ -579,6 +579,64 @@ void fuse_chain_reductions(Builder& b) {
   }
 }
 
+// The sum of a row's exponentials relative to its maximum, `>ij~i`, `ij-i~ij`, `^ij~ij`, `+ij~i`, where
+// the middle two already run inside the fold: the maximum and the sum come out of one read of x.
+// Unary maps on the sum (`$i~i`) with no other reader of it go along.  A maximum that something else
+// reads keeps its own fold.
+void fuse_row_expsum(Builder& b) {
+  for (size_t n = 0; n < b.g.nodes.size(); ++n) {
+    if (!b.alive[n]) continue;
+    const Step& red = b.steps[n];
+    if (red.kind != StepKind::ChainReduce || red.op != Op::Add || red.in.size() != 2 || red.chain.size() != 2)
+      continue;
+    const ChainOp &shift = red.chain[0], &power = red.chain[1];
+    if (shift.op != Op::Sub || shift.lhs != 0 || shift.rhs != 1 || power.op != Op::Pow ||
+        power.lhs != kChainPrev || power.rhs != kChainNone)
+      continue;
+    if (!is_iota(red.in[0].index, red.rank) || !is_iota(red.in[1].index, red.rank - 1)) continue;
+    if (red.in[1].buffer.is_input) continue;
+    const size_t m_node = red.in[1].buffer.index;
+    if (!b.alive[m_node] || !is_row_reduce(b.steps[m_node], Op::Max)) continue;
+    const Step& mx = b.steps[m_node];
+    if (!(mx.in[0].buffer == red.in[0].buffer) || mx.rank != red.rank) continue;
+
+    Step fused;
+    fused.kind = StepKind::RowExpSum;
+    fused.op = Op::Add;
+    fused.rank = red.rank;
+    fused.in = {red.in[0]};
+    fused.out = red.out;
+    fused.hint = red.hint;
+    fused.nodes = red.nodes;
+    if (auto only = b.sole_reader(m_node); only && *only == n) {
+      fused.nodes.insert(fused.nodes.begin(), mx.nodes.begin(), mx.nodes.end());
+      b.alive[m_node] = false;
+    }
+    size_t slot = n;
+    for (;;) {
+      auto reader = b.sole_reader(fused.out.buffer.index);
+      if (!reader || fused.chain.size() >= kMaxChainOps) break;
+      const Step& next = b.steps[*reader];
+      if ((next.kind != StepKind::Map && next.kind != StepKind::MapChain) || next.in.size() != 1 ||
+          next.rank + 1 != fused.rank || !is_iota(next.in[0].index, next.rank) || !is_iota(next.out.index, next.rank))
+        break;
+      std::vector<ChainOp> ops = next.chain;
+      if (next.kind == StepKind::Map) ops = {ChainOp{next.op, 0, kChainNone}};
+      bool unary = fused.chain.size() + ops.size() <= kMaxChainOps;
+      for (size_t j = 0; unary && j < ops.size(); ++j)
+        unary = ops[j].rhs == kChainNone && ops[j].lhs == (j == 0 ? 0 : kChainPrev);
+      if (!unary) break;
+      for (const ChainOp& c : ops) fused.chain.push_back(ChainOp{c.op, kChainPrev, kChainNone});
+      fused.out = next.out;
+      fused.nodes.insert(fused.nodes.end(), next.nodes.begin(), next.nodes.end());
+      b.alive[slot] = false;
+      slot = *reader;
+      b.steps[slot] = fused;
+    }
+    b.steps[slot] = std::move(fused);
+  }
+}
+
 // A contraction whose only reader is a pointwise map or chain over the same index space, built
 // from `+ - * > <` (a bias, a scale, a rectifier) with the contraction's result as the value the
 // chain starts from: the operators run in the contraction's epilogue, on the accumulator, and the
@@ -594,7 +652,7 @@ void fuse_contract_epilogues(Builder& b) {
     if (!b.alive[n]) continue;
     const Step& con = b.steps[n];
     if (con.kind != StepKind::Contract || !con.chain.empty()) continue;
-    if (con.form.swap_out || !con.form.has_m || !con.form.has_n) continue;
+    if (con.form.swap_out || (!con.form.has_m && !con.form.has_n)) continue;
     const size_t c_node = con.out.buffer.index;
     auto reader = b.sole_reader(c_node);
     if (!reader) continue;
@@ -662,6 +720,7 @@ const char* kind_name(StepKind k) {
     case StepKind::ChainReduce: return "chain_reduce";
     case StepKind::Reduce: return "reduce";
     case StepKind::Contract: return "contract";
+    case StepKind::RowExpSum: return "row_expsum";
     case StepKind::RowSoftmax: return "row_softmax";
     case StepKind::Attention: return "attention";
   }
@@ -716,6 +775,11 @@ std::string Plan::describe() const {
           }
           os << "\n";
         }
+        break;
+      case StepKind::RowExpSum:
+        os << "    kernel: ib_row_expsum (maximum and sum of exponentials in one read)";
+        for (const ChainOp& c : s.chain) os << "  " << op_token(c.op) << "_";
+        os << "\n";
         break;
       case StepKind::RowSoftmax:
         os << "    kernel: ib_row_softmax (row resident on chip, one read + one write)\n";
@@ -831,6 +895,7 @@ Result<Plan> make_plan(const Graph& g) {
   fuse_deferred_attention(b);
   fuse_map_chains(b);
   fuse_chain_reductions(b);
+  fuse_row_expsum(b);
   fuse_contract_epilogues(b);
 
   Plan plan;

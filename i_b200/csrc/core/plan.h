@@ -22,6 +22,7 @@ enum class StepKind {
   ChainReduce,  // the same, folded along the last axis instead of stored (Step::op is the fold)
   Reduce,       // fold over the axes missing from the output
   Contract,     // Mul node + Add-reduce node = batched GEMM
+  RowExpSum,    // max, shift, exp, sum over the last axis (then `chain`, unary operators on the sum)
   RowSoftmax,   // max, shift, exp, sum, divide over the last axis
   Attention     // Contract -> RowSoftmax -> Contract, fused online softmax
 };

@@ -509,7 +509,9 @@ int run_contract(const Step& step, const std::vector<size_t>& extent, DeviceBuff
   const float* a = dev.get(step.in[0].buffer);
   const float* b = dev.get(step.in[1].buffer);
   bool a_kmajor = f.a_kmajor, b_kmajor = f.b_kmajor;
-  if (f.swap_out) {  // result stored [n][m]: compute B A^T instead
+  // Result stored [n][m]: compute B A^T instead.  A result without a column axis is taken as one row
+  // per batch entry, which is how operators on it address their operands.
+  if (f.swap_out || (f.has_m && !f.has_n)) {
     std::swap(a, b);
     std::swap(m, n);
     std::swap(a_kmajor, b_kmajor);
@@ -613,6 +615,14 @@ int run_plan(const i_program* program, const ShapeTable& shapes, const float* co
       case StepKind::ChainReduce: rc = run_map_chain(step, shapes, dev, out, oshape); break;
       case StepKind::Reduce: rc = run_reduce(step, shapes, extent, dev, out, oshape); break;
       case StepKind::Contract: rc = run_contract(step, extent, dev, out, precision, &err); break;
+      case StepKind::RowExpSum: {
+        const Shape& xs = *shapes.get(step.in[0].buffer);
+        int post[IB_MAX_CHAIN_OPS];
+        for (size_t c = 0; c < step.chain.size(); ++c) post[c] = op_code(step.chain[c].op);
+        rc = ib_row_expsum(dev.get(step.in[0].buffer), out, product(oshape), xs.back(),
+                           static_cast<int>(step.chain.size()), post, stream);
+        break;
+      }
       case StepKind::RowSoftmax: {
         const Shape& xs = *shapes.get(step.in[0].buffer);
         size_t cols = xs.empty() ? 1 : xs.back();

@@ -13,7 +13,9 @@
 //
 // Results too few for the machine: a product is cut along k into up to eight parts, the CTAs of one
 // cluster, whose sums meet in distributed shared memory: no workspace, no second launch, a fixed
-// order.  Tile and parts are chosen by an estimate (choose below).
+// order.  Tile and parts are chosen by an estimate (choose below).  Where even eight parts leave SMs
+// idle on a deep product, several clusters take a tile and their sums go through copies of the result
+// (fp32_copies).
 //
 // Measured on B200, against 64 x 64 tiles of 4 x 4 results with 4-byte shared-memory reads: 1024 x
 // 1000 x 1001 145 -> 62 us, 2048 x 2048 x 512 105 us (41 TFLOP/s; the FMA pipe is 66-69 % busy, held
@@ -40,7 +42,7 @@ struct Fp32Args {
   Operand a, b;
   float* c;
   size_t k, k_len;
-  unsigned tiles_n, parts;
+  unsigned tiles_n, parts, copies;         // blockIdx.y = batch entry * copies + copy
   bool c_vec;
 };
 
@@ -166,10 +168,10 @@ contract_fp32_kernel(const __grid_constant__ Fp32Args g, const __grid_constant__
 
   const unsigned tile = blockIdx.x / g.parts, part = blockIdx.x - tile * g.parts;
   const size_t i0 = static_cast<size_t>(tile / g.tiles_n) * BM, j0 = static_cast<size_t>(tile % g.tiles_n) * BN;
-  const size_t m = g.a.rows, n = g.b.rows, batch = blockIdx.y;
+  const size_t m = g.a.rows, n = g.b.rows, out = blockIdx.y, batch = out / g.copies;
   const float* a = g.a.p + batch * m * g.k;
   const float* b = g.b.p + batch * n * g.k;
-  const size_t k_lo = part * g.k_len, k_hi = k_lo + g.k_len < g.k ? k_lo + g.k_len : g.k;
+  const size_t k_lo = ((out - batch * g.copies) * g.parts + part) * g.k_len, k_hi = k_lo + g.k_len < g.k ? k_lo + g.k_len : g.k;
   const int tx = threadIdx.x % kAcross, ty = threadIdx.x / kAcross;
 
   unsigned long long acc[TM][TN / 2];
@@ -228,7 +230,7 @@ contract_fp32_kernel(const __grid_constant__ Fp32Args g, const __grid_constant__
 #pragma unroll
       for (int q = 0; q < kQn; ++q) {
         const float2 lo = halves(acc[u][2 * q]), hi = halves(acc[u][2 * q + 1]);
-        put_quad(g.c, make_float4(lo.x, lo.y, hi.x, hi.y), batch * m + gi, j0 + q * (BN / kQn) + tx * 4, n, g.c_vec,
+        put_quad(g.c, make_float4(lo.x, lo.y, hi.x, hi.y), out * m + gi, j0 + q * (BN / kQn) + tx * 4, n, g.c_vec,
                  epilogue);
       }
     }
@@ -260,7 +262,7 @@ contract_fp32_kernel(const __grid_constant__ Fp32Args g, const __grid_constant__
         if (p < g.parts) {
           sum.x += x[p].x; sum.y += x[p].y; sum.z += x[p].z; sum.w += x[p].w;
         }
-      put_quad(g.c, sum, batch * m + gi, gj, n, g.c_vec, epilogue);
+      put_quad(g.c, sum, out * m + gi, gj, n, g.c_vec, epilogue);
     }
     cluster.sync();                          // nobody leaves while its shared memory is read
   }
@@ -303,21 +305,23 @@ Choice choose(size_t batch, size_t m, size_t n, size_t k) {
 }
 
 template <int BM, int BN, int TK, int TM, int TN>
-cudaError_t launch_tile(Fp32Args g, const GemmEpilogue& e, size_t batch, size_t parts, bool ak, bool bk,
-                        cudaStream_t s) {
+cudaError_t launch_tile(Fp32Args g, const GemmEpilogue& e, size_t batch, size_t parts, size_t copies, bool ak,
+                        bool bk, cudaStream_t s) {
   const size_t tiles_m = (g.a.rows + BM - 1) / BM, tiles_n = (g.b.rows + BN - 1) / BN;
   const size_t ctas = tiles_m * tiles_n * parts;
   if (ctas > 0x7fffffffu || tiles_n > 0x7fffffffu) return cudaErrorInvalidConfiguration;
   g.tiles_n = static_cast<unsigned>(tiles_n);
   g.parts = static_cast<unsigned>(parts);
-  // Whole k-tiles per part, so that every part but the last is full.
-  g.k_len = ((g.k + parts - 1) / parts + TK - 1) / TK * TK;
+  g.copies = static_cast<unsigned>(copies);
+  // Whole k-tiles per part, so that every part but the last ones is full.
+  const size_t cuts = parts * copies;
+  g.k_len = ((g.k + cuts - 1) / cuts + TK - 1) / TK * TK;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = static_cast<unsigned>(parts);
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(ctas), static_cast<unsigned>(batch));
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas), static_cast<unsigned>(batch * copies));
   cfg.blockDim = dim3((BM / TM) * (BN / TN));
   cfg.stream = s;
   cfg.attrs = &attr;
@@ -330,33 +334,49 @@ cudaError_t launch_tile(Fp32Args g, const GemmEpilogue& e, size_t batch, size_t 
 
 }  // namespace
 
+// Copies of the result a deep product with few tiles is summed into (1 = none): two CTAs per SM, at
+// least 128 terms each.  The copies cost a second launch (3-4 us with the fold), so only where they
+// halve the chain of a part: 30 x 257 x 12288 on B200 43 us with one cluster per tile.
+size_t fp32_copies(size_t batch, size_t m, size_t n, size_t k) {
+  const Choice pick = choose(batch, m, n, k);
+  if (pick.parts != static_cast<size_t>(kMaxParts)) return 1;
+  const TileShape& s = kTiles[pick.tile];
+  const size_t ctas = batch * ((m + s.bm - 1) / s.bm) * ((n + s.bn - 1) / s.bn) * pick.parts;
+  size_t copies = 2 * static_cast<size_t>(kNumSMs) / ctas;
+  if (copies > k / (pick.parts * 128)) copies = k / (pick.parts * 128);
+  if (copies > 16) copies = 16;
+  if (batch * copies > 65535) return 1;
+  return copies < 2 ? 1 : copies;
+}
+
 int contract_fp32(const float* a, const float* b, float* c, size_t batch, size_t m, size_t n, size_t k,
-                  bool a_kmajor, bool b_kmajor, cudaStream_t s, const GemmEpilogue* e) {
+                  bool a_kmajor, bool b_kmajor, cudaStream_t s, const GemmEpilogue* e, float* copies) {
   if (batch == 0 || m == 0 || n == 0) return 0;
   if (batch > 65535) return fail("ib_contract: more than 65535 batch entries");
   // 16-byte loads need every row of the operand, in every batch entry, to start on 16 bytes.
   Fp32Args g{};
   g.a = Operand{a, m, (a_kmajor ? k : m) % 4 == 0 && aligned16(a)};
   g.b = Operand{b, n, (b_kmajor ? k : n) % 4 == 0 && aligned16(b)};
-  g.c = c;
+  const size_t n_copies = copies ? fp32_copies(batch, m, n, k) : 1;
+  g.c = n_copies > 1 ? copies : c;
   g.k = k;
-  g.c_vec = n % 4 == 0 && aligned16(c);
+  g.c_vec = n % 4 == 0 && aligned16(g.c);
   const Choice pick = choose(batch, m, n, k);
   const GemmEpilogue none{};
-  const GemmEpilogue& ep = e ? *e : none;
+  const GemmEpilogue& ep = e && n_copies == 1 ? *e : none;
   cudaError_t err;
   switch (pick.tile) {
-    case 0: err = launch_tile<128, 128, 16, 8, 8>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
-    case 1: err = launch_tile<64, 128, 16, 8, 8>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
-    case 2: err = launch_tile<64, 64, 32, 8, 4>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
-    default: err = launch_tile<32, 32, 32, 4, 4>(g, ep, batch, pick.parts, a_kmajor, b_kmajor, s); break;
+    case 0: err = launch_tile<128, 128, 16, 8, 8>(g, ep, batch, pick.parts, n_copies, a_kmajor, b_kmajor, s); break;
+    case 1: err = launch_tile<64, 128, 16, 8, 8>(g, ep, batch, pick.parts, n_copies, a_kmajor, b_kmajor, s); break;
+    case 2: err = launch_tile<64, 64, 32, 8, 4>(g, ep, batch, pick.parts, n_copies, a_kmajor, b_kmajor, s); break;
+    default: err = launch_tile<32, 32, 32, 4, 4>(g, ep, batch, pick.parts, n_copies, a_kmajor, b_kmajor, s); break;
   }
   if (err != cudaSuccess) {
     cudaGetLastError();
     return fail(std::string("ib_contract (fp32): ") + cudaGetErrorString(err));
   }
   count_launch();
-  return 0;
+  return n_copies > 1 ? sum_partials(copies, c, batch, n_copies, m * n, s) : 0;
 }
 
 }  // namespace ib

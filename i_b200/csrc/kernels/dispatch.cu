@@ -229,7 +229,11 @@ extern "C" size_t ib_contract_workspace_bytes(size_t batch, size_t m, size_t n, 
     return carve_bytes(long_rows_floats(batch, k));   // dot products of few, very long rows
   }
   const double flop = 2.0 * batch * m * n * k;
-  if (!wants_tensor(precision, flop)) return 0;
+  const size_t fp32_bytes = [&] {
+    const size_t copies = fp32_copies(batch, m, n, k);
+    return copies > 1 ? carve_bytes(batch * copies * m * n) : 0;
+  }();
+  if (!wants_tensor(precision, flop)) return fp32_bytes;
   if (precision == IB_PRECISION_AUTO && contract_prefers_f16(m, n, k)) precision = IB_PRECISION_F16;
   if (precision == IB_PRECISION_F16) {
     // fp16 copies of both operands plus one scale per row; fp32 transposes first when needed.
@@ -248,7 +252,7 @@ extern "C" size_t ib_contract_workspace_bytes(size_t batch, size_t m, size_t n, 
     if (!b_kmajor) bytes += carve_bytes(batch * n * k);
     return bytes;
   }
-  if (!contract_shape_ok(k)) return 0;
+  if (!contract_shape_ok(k)) return fp32_bytes;
   // Copies of the result when the k range is cut into parts.
   const size_t parts = k_parts_tensor(batch, m, n, k);
   size_t bytes = parts > 1 ? carve_bytes(batch * parts * m * n) : 0;
@@ -286,8 +290,9 @@ namespace ib {
 namespace {
 
 // Pointwise operators that follow a contraction, in the two forms it needs: `fused` for the tile
-// kernels' epilogue, and the same list as an ib_map_chain call over the stored result for the routes
-// that have no epilogue hook (folds, parts added afterwards, and a contraction over no terms).
+// kernels' epilogue and the folds' last step, and the same list as an ib_map_chain call over the stored
+// result for the routes that have no such hook (one column per row, parts added afterwards, a
+// contraction over no terms).
 struct ContractChain {
   GemmEpilogue fused;
   int n_ops = 0;
@@ -416,14 +421,14 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
                                   (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0
                               ? static_cast<float*>(workspace)
                               : nullptr;
-        rc = dot_rows(a, b, false, c, batch, k, s, partials);
+        rc = dot_rows(a, b, false, c, batch, k, s, partials, fused);
       } else {
         const size_t rows = a_rows ? m : n;
         for (size_t e = 0; e < batch && rc == 0; ++e)
           rc = dot_rows((a_rows ? a : b) + e * rows * k, (a_rows ? b : a) + e * k, true, c + e * rows,
-                        rows, k, s);
+                        rows, k, s, nullptr, b_rows ? fused : nullptr, e);
       }
-      return then_chain(rc);
+      return b_rows || dots ? rc : then_chain(rc);
     }
     // The same with the matrix stored k-major the other way round, [k][rows]: vector times
     // matrix, a weighted fold down the columns.
@@ -439,8 +444,8 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
       int rc = 0;
       for (size_t e = 0; e < batch && rc == 0; ++e)
         rc = dot_leading_axis((a_cols ? a : b) + e * k * cols, (a_cols ? b : a) + e * k, c + e * cols, k,
-                              cols, partials, s);
-      return then_chain(rc);
+                              cols, partials, s, b_cols ? fused : nullptr, e);
+      return b_cols ? rc : then_chain(rc);
     }
   }
   const double flop = 2.0 * batch * m * n * k;
@@ -536,7 +541,13 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
     // Misaligned base pointers: the fp32 arm takes any layout.
     return contract_fp32(ak, bk, c, batch, m, n, k, true, true, s, fused);
   }
-  return contract_fp32(a, b, c, batch, m, n, k, a_kmajor != 0, b_kmajor != 0, s, fused);
+  const size_t n_copies = fp32_copies(batch, m, n, k);
+  Carver ws(workspace, workspace_bytes);
+  float* copies = n_copies > 1 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0
+                      ? ws.take(batch * n_copies * m * n)
+                      : nullptr;
+  const int rc = contract_fp32(a, b, c, batch, m, n, k, a_kmajor != 0, b_kmajor != 0, s, fused, copies);
+  return copies ? then_chain(rc) : rc;
 }
 
 }  // namespace

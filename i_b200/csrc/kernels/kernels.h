@@ -10,6 +10,21 @@
 
 namespace ib {
 
+// Pointwise operators a contraction applies to every element of its result before
+// storing it (a bias, a rectifier, a scale), in order: acc = op(acc, other), op(other, acc) with
+// acc_right, or the one-operand form op(acc) with which < 0.  `other` is operand[which], addressed
+// by mode 0 [row][col] (the result's own shape, batch entries flattened into rows), 1 [row],
+// 2 [col], 3 one value.  Operators: IB_OP_ADD, IB_OP_SUB, IB_OP_MUL, IB_OP_MAX, IB_OP_MIN, with
+// the arithmetic of the pointwise kernels, so the result equals contraction then maps bit for bit.
+struct GemmEpilogue {
+  int n_ops = 0;
+  int op[IB_MAX_CHAIN_OPS] = {};
+  int which[IB_MAX_CHAIN_OPS] = {};
+  int acc_right[IB_MAX_CHAIN_OPS] = {};
+  const float* operand[IB_MAX_CHAIN_OPERANDS] = {};
+  int mode[IB_MAX_CHAIN_OPERANDS] = {};
+};
+
 // reduce.cu
 // y[b][c] = sum_r x[b][r][c] for a handful of rows (the copies of a split contraction).
 int sum_partials(const float* x, float* y, size_t batch, size_t rows, size_t cols, cudaStream_t s);
@@ -33,15 +48,16 @@ int prepare_attention_operands(const float* q, float* qr, size_t q_elems, const 
 // reduce.cu — y[r] = sum_c x[r][c] * w[r][c], or x[r][c] * w[c] with w_is_vector: row-wise dot
 // products and matrix times vector as one pass over memory (products rounded, then a tree sum).
 // Few rows of very many columns are folded in segments; `partials` then holds long_rows_floats
-// floats (null: every row is folded whole).
+// floats (null: every row is folded whole).  The operators of `e` are applied to the results, which
+// are row `out_row` of the contraction's result (vector) or one row each (row-wise).
 size_t long_rows_floats(size_t rows, size_t cols);
 int dot_rows(const float* x, const float* w, bool w_is_vector, float* y, size_t rows, size_t cols,
-             cudaStream_t s, float* partials = nullptr);
+             cudaStream_t s, float* partials = nullptr, const GemmEpilogue* e = nullptr, size_t out_row = 0);
 // y[c] = sum_r x[r][c] * w[r] (vector times matrix); `partials` holds dot_leading_axis_floats
 // floats (null: the rows are folded as one slab).
 size_t dot_leading_axis_floats(size_t rows, size_t cols);
 int dot_leading_axis(const float* x, const float* w, float* y, size_t rows, size_t cols,
-                     float* partials, cudaStream_t s);
+                     float* partials, cudaStream_t s, const GemmEpilogue* e = nullptr, size_t out_row = 0);
 
 // device_util.cu — encodes a TMA descriptor for a dense fp32 tensor
 // [batch][rows][cols] (cols contiguous, `row_pitch` elements between rows) read
@@ -71,24 +87,14 @@ struct GemmGeometry {
   int col_tile = 0;
   int group_n = 0;
 };
-// Pointwise operators the tensor-core contraction applies to every element of its result before
-// storing it (a bias, a rectifier, a scale), in order: acc = op(acc, other), op(other, acc) with
-// acc_right, or the one-operand form op(acc) with which < 0.  `other` is operand[which], addressed
-// by mode 0 [row][col] (the result's own shape, batch entries flattened into rows), 1 [row],
-// 2 [col], 3 one value.  Operators: IB_OP_ADD, IB_OP_SUB, IB_OP_MUL, IB_OP_MAX, IB_OP_MIN, with
-// the arithmetic of the pointwise kernels, so the result equals contraction then maps bit for bit.
-struct GemmEpilogue {
-  int n_ops = 0;
-  int op[IB_MAX_CHAIN_OPS] = {};
-  int which[IB_MAX_CHAIN_OPS] = {};
-  int acc_right[IB_MAX_CHAIN_OPS] = {};
-  const float* operand[IB_MAX_CHAIN_OPERANDS] = {};
-  int mode[IB_MAX_CHAIN_OPERANDS] = {};
-};
 // contract_fp32.cu — the contraction in fp32 on the CUDA cores, any extents and layouts, with the
-// operators of `e` applied before the store.
+// operators of `e` applied before the store.  With `copies` (batch * fp32_copies * m * n floats, where
+// that count is above 1) a deep product with few tiles sums into so many copies, adds them, and
+// leaves the operators to the caller.
+size_t fp32_copies(size_t batch, size_t m, size_t n, size_t k);
 int contract_fp32(const float* a, const float* b, float* c, size_t batch, size_t m, size_t n,
-                  size_t k, bool a_kmajor, bool b_kmajor, cudaStream_t s, const GemmEpilogue* e = nullptr);
+                  size_t k, bool a_kmajor, bool b_kmajor, cudaStream_t s, const GemmEpilogue* e = nullptr,
+                  float* copies = nullptr);
 // k_parts > 1 (one batch entry, k a multiple of 4 * k_parts): the k range is cut into that many
 // equal parts and c receives one copy of the result per part, [part][m][n], for the caller to add.
 int gemm_tcgen05(const float* a, const float* b, float* c, size_t batch, size_t m, size_t n,

@@ -9,6 +9,8 @@
 // flight per thread and one CTA per row (no cap on the grid) measured 5.6-5.85 TB/s on B200 against
 // 5.2 for two loads per thread on a grid capped at 16 CTAs per SM.
 #include "common.cuh"
+#include "epilogue.cuh"
+#include "kernels.h"
 
 namespace ib {
 namespace {
@@ -30,6 +32,18 @@ constexpr int kUnroll = IB_RED_UNROLL;   // 16-byte loads in flight per thread i
 // c = c + tmp` is (ilang-python/annotated-flashattn.c:67-85).
 enum Weight { kPlain, kTimesRows, kTimesVector };
 
+// Pointwise operators on the results of a contraction that runs as folds: result number i is element
+// [row][i] of a result `cols` wide, or element [i][0] when cols is 0.
+struct Post {
+  GemmEpilogue e;
+  size_t row = 0, cols = 0;
+};
+template <bool POST>
+__device__ __forceinline__ float finished(const Post& p, float v, size_t i) {
+  if (!POST) return v;
+  return p.cols ? epilogue_value(p.e, v, p.row, i, p.cols) : epilogue_value(p.e, v, i, 0, 1);
+}
+
 template <int WEIGHT>
 __device__ __forceinline__ float4 weighted(float4 v, const float4* w_row4, const float4* w_vec4, size_t i) {
   if (WEIGHT == kPlain) return v;
@@ -37,10 +51,10 @@ __device__ __forceinline__ float4 weighted(float4 v, const float4* w_row4, const
   return make_float4(__fmul_rn(v.x, w.x), __fmul_rn(v.y, w.y), __fmul_rn(v.z, w.z), __fmul_rn(v.w, w.w));
 }
 
-template <int OP, int WEIGHT = kPlain>
+template <int OP, int WEIGHT = kPlain, bool POST = false>
 __global__ void __launch_bounds__(kThreads)
 reduce_rows_warp(const float* __restrict__ x, float* __restrict__ y, size_t rows, size_t cols,
-                 bool vec, const float* __restrict__ w = nullptr) {
+                 bool vec, const float* __restrict__ w, const __grid_constant__ Post post) {
   const int lane = threadIdx.x & 31;
   const size_t warps_total = static_cast<size_t>(gridDim.x) * kWarps;
   if (vec && cols <= 128) {
@@ -66,7 +80,7 @@ reduce_rows_warp(const float* __restrict__ x, float* __restrict__ y, size_t rows
 #pragma unroll
       for (int u = 0; u < kRowsAtOnce; ++u) {
         const float total = warp_fold<OP>(acc[u]);
-        if (lane == 0 && r0 + u < rows) y[r0 + u] = total;
+        if (lane == 0 && r0 + u < rows) y[r0 + u] = finished<POST>(post, total, r0 + u);
       }
     }
     return;
@@ -100,7 +114,7 @@ reduce_rows_warp(const float* __restrict__ x, float* __restrict__ y, size_t rows
         acc = fold<OP>(acc, WEIGHT == kPlain ? row[i] : __fmul_rn(row[i], wrow[i]));
     }
     acc = warp_fold<OP>(acc);
-    if (lane == 0) y[r] = acc;
+    if (lane == 0) y[r] = finished<POST>(post, acc, r);
   }
 }
 
@@ -108,10 +122,11 @@ reduce_rows_warp(const float* __restrict__ x, float* __restrict__ y, size_t rows
 // A row may be cut into `segs` segments of `seg_len` columns (a multiple of four; the last one
 // shorter), each folded by a CTA of its own into y[row * segs + segment]: few rows of millions of
 // columns (a sum over a whole array) would otherwise keep one CTA each busy and the rest idle.
-template <int OP, int WEIGHT = kPlain>
+template <int OP, int WEIGHT = kPlain, bool POST = false>
 __global__ void __launch_bounds__(kThreads)
 reduce_rows_block(const float* __restrict__ x, float* __restrict__ y, size_t rows, size_t cols,
-                  bool vec, const float* __restrict__ w = nullptr, size_t segs = 1, size_t seg_len = 0) {
+                  bool vec, const float* __restrict__ w, size_t segs, size_t seg_len,
+                  const __grid_constant__ Post post) {
   __shared__ float partial[kWarps];
   for (size_t r = blockIdx.x; r < rows * segs; r += gridDim.x) {
     const size_t whole = r / segs, at = (r - whole * segs) * seg_len;
@@ -152,7 +167,7 @@ reduce_rows_block(const float* __restrict__ x, float* __restrict__ y, size_t row
     if (threadIdx.x < 32) {
       float v = threadIdx.x < kWarps ? partial[threadIdx.x] : reduce_identity(OP);
       v = warp_fold<OP>(v);
-      if (threadIdx.x == 0) y[r] = v;
+      if (threadIdx.x == 0) y[r] = finished<POST>(post, v, r);
     }
     __syncthreads();
   }
@@ -215,19 +230,19 @@ RowSplit split_long_rows(size_t rows, size_t cols) {
   return sp;
 }
 
-template <int OP, int WEIGHT>
+template <int OP, int WEIGHT, bool POST = false>
 int launch_rows_split(const float* x, const float* w, float* y, size_t rows, size_t cols, float* partials,
-                      cudaStream_t s) {
+                      cudaStream_t s, const Post& post = {}) {
   const RowSplit sp = split_long_rows(rows, cols);
   const bool vec = cols % 4 == 0 && aligned16(x) && (WEIGHT == kPlain || aligned16(w));
   const size_t cap = static_cast<size_t>(kNumSMs) * IB_RED_CAP;
   const size_t ctas = rows * sp.segs;
   reduce_rows_block<OP, WEIGHT><<<static_cast<int>(ctas < cap ? ctas : cap), kThreads, 0, s>>>(
-      x, partials, rows, cols, vec, w, sp.segs, sp.seg_len);
+      x, partials, rows, cols, vec, w, sp.segs, sp.seg_len, Post{});
   if (int rc = check_launch("ib_reduce_rows (segments)")) return rc;
   const size_t blocks = (rows + kWarps - 1) / kWarps;
-  reduce_rows_warp<OP><<<static_cast<int>(blocks < cap ? blocks : cap), kThreads, 0, s>>>(
-      partials, y, rows, sp.segs, sp.segs % 4 == 0 && aligned16(partials));
+  reduce_rows_warp<OP, kPlain, POST><<<static_cast<int>(blocks < cap ? blocks : cap), kThreads, 0, s>>>(
+      partials, y, rows, sp.segs, sp.segs % 4 == 0 && aligned16(partials), nullptr, post);
   return check_launch("ib_reduce_rows (partials)");
 }
 
@@ -241,29 +256,29 @@ int launch_rows(const float* x, float* y, size_t rows, size_t cols, cudaStream_t
     size_t blocks = (rows + kWarps - 1) / kWarps;
     size_t cap = static_cast<size_t>(kNumSMs) * IB_RED_CAP;
     reduce_rows_warp<OP><<<static_cast<int>(blocks < cap ? blocks : cap), kThreads, 0, s>>>(
-        x, y, rows, cols, vec);
+        x, y, rows, cols, vec, nullptr, Post{});
   } else {
     size_t cap = static_cast<size_t>(kNumSMs) * IB_RED_CAP;
     reduce_rows_block<OP><<<static_cast<int>(rows < cap ? rows : cap), kThreads, 0, s>>>(
-        x, y, rows, cols, vec);
+        x, y, rows, cols, vec, nullptr, 1, 0, Post{});
   }
   return check_launch("ib_reduce_rows");
 }
 
-template <int WEIGHT>
+template <int WEIGHT, bool POST>
 int launch_dot_rows(const float* x, const float* w, float* y, size_t rows, size_t cols, cudaStream_t s,
-                    float* partials) {
+                    float* partials, const Post& post) {
   if (partials && split_long_rows(rows, cols).segs > 1)
-    return launch_rows_split<IB_OP_ADD, WEIGHT>(x, w, y, rows, cols, partials, s);
+    return launch_rows_split<IB_OP_ADD, WEIGHT, POST>(x, w, y, rows, cols, partials, s, post);
   const bool vec = cols % 4 == 0 && aligned16(x) && aligned16(w);
   const size_t cap = static_cast<size_t>(kNumSMs) * IB_RED_CAP;
   if (cols <= 2048) {
     const size_t blocks = (rows + kWarps - 1) / kWarps;
-    reduce_rows_warp<IB_OP_ADD, WEIGHT><<<static_cast<int>(blocks < cap ? blocks : cap), kThreads, 0, s>>>(
-        x, y, rows, cols, vec, w);
+    reduce_rows_warp<IB_OP_ADD, WEIGHT, POST><<<static_cast<int>(blocks < cap ? blocks : cap), kThreads, 0, s>>>(
+        x, y, rows, cols, vec, w, post);
   } else {
-    reduce_rows_block<IB_OP_ADD, WEIGHT><<<static_cast<int>(rows < cap ? rows : cap), kThreads, 0, s>>>(
-        x, y, rows, cols, vec, w);
+    reduce_rows_block<IB_OP_ADD, WEIGHT, POST><<<static_cast<int>(rows < cap ? rows : cap), kThreads, 0, s>>>(
+        x, y, rows, cols, vec, w, 1, 0, post);
   }
   return check_launch("ib_contract (rows)");
 }
@@ -280,10 +295,11 @@ int launch_dot_rows(const float* x, const float* w, float* y, size_t rows, size_
 // is added).  Algorithmic traffic: rows*cols*4 + cols*4 bytes.
 constexpr int kColsUnroll = 8;
 
-template <int OP, bool ROW_WEIGHT, bool VEC>
+template <int OP, bool ROW_WEIGHT, bool VEC, bool POST = false>
 __global__ void __launch_bounds__(kThreads)
 fold_leading_axis(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
-                  size_t rows, size_t cols, size_t rows_per_slab, int lanes_log2) {
+                  size_t rows, size_t cols, size_t rows_per_slab, int lanes_log2,
+                  const __grid_constant__ Post post) {
   constexpr int kWidth = VEC ? 4 : 1;
   __shared__ float meet[kThreads][kWidth];
   // blockIdx.z: one of several arrays of the same shape, one behind the other (`+bij~bj`).
@@ -343,6 +359,10 @@ fold_leading_axis(const float* __restrict__ x, const float* __restrict__ w, floa
       for (int e = 0; e < kWidth; ++e) acc[e] = fold<OP>(acc[e], meet[p * lanes + tx][e]);
   }
   if (!live) return;
+  if (POST) {
+#pragma unroll
+    for (int e = 0; e < kWidth; ++e) acc[e] = finished<POST>(post, acc[e], c + e);
+  }
   float* dst = y + static_cast<size_t>(blockIdx.y) * cols + c;
   if (VEC) {
     *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[kWidth > 1 ? 1 : 0], acc[kWidth > 2 ? 2 : 0],
@@ -375,9 +395,10 @@ size_t leading_axis_slabs(size_t rows, size_t cols, size_t batch = 1) {
   return slabs < 1 ? 1 : slabs;
 }
 
-template <int OP, bool ROW_WEIGHT>
+template <int OP, bool ROW_WEIGHT, bool POST = false>
 int launch_leading_axis_once(const float* x, const float* w, float* y, size_t rows, size_t cols,
-                             size_t rows_per_slab, size_t slabs, cudaStream_t s, size_t batch = 1) {
+                             size_t rows_per_slab, size_t slabs, cudaStream_t s, size_t batch = 1,
+                             const Post& post = {}) {
   const bool vec = cols % 4 == 0 && aligned16(x) && aligned16(y);
   int l = leading_axis_lanes_log2(cols, vec);
   const size_t groups = vec ? cols / 4 : cols;
@@ -392,26 +413,26 @@ int launch_leading_axis_once(const float* x, const float* w, float* y, size_t ro
   dim3 grid(static_cast<unsigned>((groups + (1u << l) - 1) >> l), static_cast<unsigned>(slabs),
             static_cast<unsigned>(batch));
   if (vec)
-    fold_leading_axis<OP, ROW_WEIGHT, true><<<grid, kThreads, 0, s>>>(x, w, y, rows, cols, rows_per_slab, l);
+    fold_leading_axis<OP, ROW_WEIGHT, true, POST><<<grid, kThreads, 0, s>>>(x, w, y, rows, cols, rows_per_slab, l, post);
   else
-    fold_leading_axis<OP, ROW_WEIGHT, false><<<grid, kThreads, 0, s>>>(x, w, y, rows, cols, rows_per_slab, l);
+    fold_leading_axis<OP, ROW_WEIGHT, false, POST><<<grid, kThreads, 0, s>>>(x, w, y, rows, cols, rows_per_slab, l, post);
   return check_launch("ib_reduce_leading");
 }
 
-template <int OP, bool ROW_WEIGHT>
+template <int OP, bool ROW_WEIGHT, bool POST = false>
 int launch_leading_axis(const float* x, const float* w, float* y, size_t rows, size_t cols,
-                        float* partials, cudaStream_t s, size_t batch = 1) {
+                        float* partials, cudaStream_t s, size_t batch = 1, const Post& post = {}) {
   if (batch > 65535) return fail("ib_reduce_leading: more than 65535 arrays");
   const size_t slabs = partials ? leading_axis_slabs(rows, cols, batch) : 1;
   const size_t rows_per_slab = (rows + slabs - 1) / slabs;
   const size_t used = rows_per_slab ? (rows + rows_per_slab - 1) / rows_per_slab : 1;   // slabs that hold rows
   if (used <= 1)
-    return launch_leading_axis_once<OP, ROW_WEIGHT>(x, w, y, rows, cols, rows ? rows : 1, 1, s, batch);
+    return launch_leading_axis_once<OP, ROW_WEIGHT, POST>(x, w, y, rows, cols, rows ? rows : 1, 1, s, batch, post);
   if (int rc = launch_leading_axis_once<OP, ROW_WEIGHT>(x, w, partials, rows, cols, rows_per_slab, used, s,
                                                         batch))
     return rc;
   // The partial rows, one per slab, folded the same way as one slab.
-  return launch_leading_axis_once<OP, false>(partials, nullptr, y, used, cols, used, 1, s, batch);
+  return launch_leading_axis_once<OP, false, POST>(partials, nullptr, y, used, cols, used, 1, s, batch, post);
 }
 
 template <int OP>
@@ -431,9 +452,21 @@ size_t dot_leading_axis_floats(size_t rows, size_t cols) {
   return slabs > 1 ? slabs * cols : 0;
 }
 
+namespace {
+Post post_of(const GemmEpilogue* e, size_t row, size_t cols) {
+  Post p;
+  if (e) p.e = *e;
+  p.row = row;
+  p.cols = cols;
+  return p;
+}
+}  // namespace
+
 int dot_leading_axis(const float* x, const float* w, float* y, size_t rows, size_t cols,
-                     float* partials, cudaStream_t s) {
+                     float* partials, cudaStream_t s, const GemmEpilogue* e, size_t out_row) {
   if (cols == 0) return 0;
+  if (e && e->n_ops)
+    return launch_leading_axis<IB_OP_ADD, true, true>(x, w, y, rows, cols, partials, s, 1, post_of(e, out_row, cols));
   return launch_leading_axis<IB_OP_ADD, true>(x, w, y, rows, cols, partials, s);
 }
 
@@ -448,10 +481,14 @@ size_t long_rows_floats(size_t rows, size_t cols) {
 }
 
 int dot_rows(const float* x, const float* w, bool w_is_vector, float* y, size_t rows, size_t cols,
-             cudaStream_t s, float* partials) {
+             cudaStream_t s, float* partials, const GemmEpilogue* e, size_t out_row) {
   if (rows == 0) return 0;
-  return w_is_vector ? launch_dot_rows<kTimesVector>(x, w, y, rows, cols, s, partials)
-                     : launch_dot_rows<kTimesRows>(x, w, y, rows, cols, s, partials);
+  if (e && e->n_ops)
+    return w_is_vector
+               ? launch_dot_rows<kTimesVector, true>(x, w, y, rows, cols, s, partials, post_of(e, out_row, rows))
+               : launch_dot_rows<kTimesRows, true>(x, w, y, rows, cols, s, partials, post_of(e, 0, 0));
+  return w_is_vector ? launch_dot_rows<kTimesVector, false>(x, w, y, rows, cols, s, partials, Post{})
+                     : launch_dot_rows<kTimesRows, false>(x, w, y, rows, cols, s, partials, Post{});
 }
 
 }  // namespace ib

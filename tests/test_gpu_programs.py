@@ -523,3 +523,62 @@ def test_concurrent_pipelined_attention_from_threads(ilang):
     for (q, k, v), o in zip(cases, outs):
         assert max_rel_to_peak(o, np_attention(q, k, v)) <= 5e-3
 
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (5, 3), (70, 130), (9, 2048), (33, 2049), (300, 5001), (2, 8192), (3, 70000), (1, 1000003)])
+def test_row_sum_of_shifted_exponentials(ilang, rows, cols):
+    # Maximum and sum of exponentials in one read: a warp, a CTA or a cluster per row, with and without
+    # 16-byte loads; unary operators on the sum; -inf among the values.  The sum is a tree of
+    # terms with 2 ulp each: 1e-5 as for the other folds of exponentials.
+    i, I = ilang.i, ilang.I
+    x = 2 * rand((rows, cols), 61)
+    if cols > 2:
+        x[:, 1] = -np.inf
+    top = x.max(axis=1, keepdims=True).astype(np.float64)
+    want = np.exp(x.astype(np.float64) - top).sum(axis=1)
+    denom = (I & i(">ij~i")) >> (i("ij-i~ij") >> i("^ij~ij") >> i("+ij~i"))
+    assert steps_of_code(denom._code()) == ["row_expsum"]
+    assert max_rel_elementwise(denom.exec_numpy(x), want) <= 1e-5
+    lse = (I & i(">ij~i")) >> (i("ij-i~ij") >> i("^ij~ij") >> i("+ij~i") >> i("$i~i") >> i("-i~i"))
+    assert steps_of_code(lse._code()) == ["row_expsum"]
+    np.testing.assert_allclose(lse.exec_numpy(x), -np.log(want), rtol=1e-5, atol=1e-6)
+    # The maximum read by something else as well: it keeps its fold, the result is the same.
+    both = (I & i(">ij~i")) >> ((i("ij-i~ij") >> i("^ij~ij") >> i("+ij~i")) & (i("ij-i~ij") >> i(">ij~i")))
+    got, zero = both.exec_numpy(x)
+    assert max_rel_elementwise(got, want) <= 1e-5 and np.array_equal(zero, np.zeros(rows, np.float32))
+
+
+def test_row_sum_of_shifted_exponentials_special_values(ilang):
+    # As in the reference's chain: a row of -inf alone and a row with +inf or NaN give NaN.
+    i, I = ilang.i, ilang.I
+    denom = (I & i(">ij~i")) >> (i("ij-i~ij") >> i("^ij~ij") >> i("+ij~i"))
+    x = np.zeros((4, 40), np.float32)
+    x[0, :] = -np.inf
+    x[1, 7] = np.inf
+    x[2, 9] = np.nan
+    got = denom.exec_numpy(x)
+    assert np.isnan(got[:3]).all() and got[3] == 40.0
+
+
+@pytest.mark.parametrize("k", [3, 1000, 4100, 70000])
+def test_operators_on_a_matrix_vector_product(ilang, k):
+    # `+ - * > <` on a result with one axis run in the fold's last step, whichever fold it is: rows by
+    # warp, by CTA, in segments, down the columns; with a vector, a scalar, the value on either side.
+    # The products are those of the plain contraction, so the results are its results, bit for bit.
+    i, I = ilang.i, ilang.I
+    rows = 5 if k == 70000 else 37
+    a, x, bias, two = rand((rows, k), 71), rand((k,), 72), rand((rows,), 73), np.float32(2.0)
+    at = np.ascontiguousarray(a.T)
+    for src, fold, args in (("ij*j~ij", "+ij~i", (a, x)), ("j*ij~ij", "+ij~i", (x, a)), ("j*ji~ji", "+ji~i", (x, at))):
+        plain = i(src) >> i(fold)
+        layer = plain >> i("i+i~i") >> i(">i~i")
+        gated = (I | plain | I) >> (i("i-i~i") | I) >> i("i*.~i")
+        assert steps_of_code(layer._code()) == steps_of_code(gated._code()) == ["contract"]
+        y = plain.exec_numpy(*args)
+        assert np.array_equal(layer.exec_numpy(*args, bias), np.maximum(y + bias, 0))
+        assert np.array_equal(gated.exec_numpy(bias, *args, two), (bias - y) * two)
+    m, s = rand((3, 20, k), 74), rand((3, k), 75)
+    plain = i("bij*bj~bij") >> i("+bij~bi")
+    shifted = plain >> i("bi+b~bi") >> i("bi*i~bi")
+    c, w = rand((3,), 76), rand((20,), 77)
+    assert np.array_equal(shifted.exec_numpy(m, s, c, w), (plain.exec_numpy(m, s) + c[:, None]) * w[None, :])
