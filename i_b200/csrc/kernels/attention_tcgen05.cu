@@ -1733,6 +1733,23 @@ long long granule_tiles(size_t kv_granule, long long kv_tiles) {
   return t < 1 ? 1 : (t > kv_tiles ? kv_tiles : t);
 }
 
+// Whether the key ranges of the row tiles that do not fill a wave are divided between the CTAs.  In
+// units of one key tile's time on an SM (1.0 - 1.2 us at d = 128): a piece of a row tile costs its key
+// tiles plus about 4 (Q staged, pipeline filled, O read out); divided, the last wave's key tiles
+// spread over all CTAs, which then handle two pieces each, write partial results and leave a merge
+// kernel to run, together about 24.  Measured on B200 (fp16 arm, back to back, divided / whole): one head of
+// 16384 170 / 164 us, of 12800 115 / 119, of 8192 66 / 81; 64 heads x 2048 276 / 262; 9 x 2048 58 / 42;
+// 40 x 700 66 / 55; 2048 queries x 16384 keys 66 / 140.
+bool divides_keys(long long units, long long kv_tiles, long long sms) {
+  constexpr double kPiece = 4.0, kDivided = 24.0;
+  const long long waves = units / sms, tail = units % sms;
+  if (tail == 0) return false;
+  const double whole = static_cast<double>(waves + 1) * (kv_tiles + kPiece);
+  const double divided = static_cast<double>(waves) * (kv_tiles + kPiece) +
+                         static_cast<double>(tail) * kv_tiles / sms + kDivided;
+  return divided < whole;
+}
+
 // SMs the persistent kernel leaves free (for a communication kernel running next to it).
 std::atomic<int> g_reserved_sms{0};
 
@@ -1826,7 +1843,9 @@ int attention_tcgen05(const float* q, const void* k, const void* vt, float* o, s
   const long long units = static_cast<long long>(p.q_tiles) * p.batch;
   // Where a row tile's key range may be cut between CTAs: at multiples of the caller's granule
   // (whole 128-key tiles); a granule of the whole range or more means never.
-  p.coarse = static_cast<int>(granule_tiles(kv_granule, p.kv_tiles));
+  p.coarse = static_cast<int>(divides_keys(units, p.kv_tiles, device_sms())
+                                  ? granule_tiles(kv_granule, p.kv_tiles)
+                                  : static_cast<long long>(p.kv_tiles));
   p.kv_coarse = (p.kv_tiles + p.coarse - 1) / p.coarse;
   const int ctas = choose_ctas(units, p.kv_tiles, p.kv_coarse, device_sms());
   p.ctas = ctas;

@@ -113,33 +113,40 @@ def set_reserved_sms(n):
     _ok(_core.i_b200_set_reserved_sms(int(n)))
 
 
-# Native marshalling of the common calls (csrc/python): {kind: module}, None where it cannot be used.
-_native = {}
+# Native marshalling of the common calls (csrc/python): the module that takes CUDA tensors, the one
+# that takes NumPy arrays; None until torch (NumPy) is in the process, False where there is none.
+_cuda_call = None
+_host_call = None
 
 
-def _native_call(kind):
-    """The extension module that makes calls with CUDA tensors ("cuda") or NumPy arrays ("host")
-    without ctypes, or None.  Loaded on first use, and only once torch (or NumPy) is in the process."""
-    needs = {"cuda": "torch", "host": "numpy"}[kind]
-    if kind not in _native:
-        if needs not in sys.modules:
-            return None
-        module = None
-        path = os.path.join(_HERE, "lib", "_%s_call.so" % kind)
-        if os.path.exists(path):
-            name = "_%s_call" % kind
-            loader = importlib.machinery.ExtensionFileLoader(name, path)
-            module = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
-            loader.exec_module(module)
-            symbols = ["i_b200_exec_into" if kind == "cuda" else "i_exec_into", "i_output_count",
-                       "i_output_ranks", "i_output_shapes", "i_error"]
-            addresses = [ctypes.cast(getattr(_core, s), _VOIDP).value for s in symbols]
-            if kind == "host":
-                import numpy as np
-                addresses += [np.ndarray, np.empty, np.float32]
-            module.bind(*addresses)
-        _native[kind] = module
-    return _native[kind]
+def _load_call(kind, needs):
+    """The extension module `_<kind>_call`, bound to the loaded library; None while the package it
+    `needs` is not in the process, False if it was not built."""
+    if needs not in sys.modules:
+        return None
+    name = "_%s_call" % kind
+    path = os.path.join(_HERE, "lib", name + ".so")
+    if not os.path.exists(path):
+        return False
+    loader = importlib.machinery.ExtensionFileLoader(name, path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
+    loader.exec_module(module)
+    symbols = ["i_b200_exec_into" if kind == "cuda" else "i_exec_into", "i_output_count",
+               "i_output_ranks", "i_output_shapes", "i_error"]
+    addresses = [ctypes.cast(getattr(_core, s), _VOIDP).value for s in symbols]
+    if kind == "host":
+        import numpy as np
+        addresses += [np.ndarray, np.empty, np.float32]
+    module.bind(*addresses)
+    return module
+
+
+def _load_calls():
+    global _cuda_call, _host_call
+    if _cuda_call is None:
+        _cuda_call = _load_call("cuda", "torch")
+    if _host_call is None:
+        _host_call = _load_call("host", "numpy")
 
 
 def _fail():
@@ -408,21 +415,23 @@ class Component:
         return outputs[0] if len(outputs) == 1 else tuple(outputs)
 
     def exec_numpy(self, *inputs):
-        import numpy as np
-        native = _native.get("host") or _native_call("host")
-        if native is not None:
-            done = native.exec(self._compiled[0] or self._compile(), inputs)
+        if _host_call is None:
+            _load_calls()
+        if _host_call:
+            done = _host_call.exec(self._compiled[0] or self._compile(), inputs)
             if done is not None:
                 return done
+        import numpy as np
         return self._run_into_new(lambda shape: np.empty(shape, dtype=np.float32), inputs)
 
     def exec_torch(self, *inputs):
-        import torch
-        native = _native.get("cuda") or _native_call("cuda")
-        if native is not None:
-            done = native.exec(self._compiled[0] or self._compile(), inputs)
+        if _cuda_call is None:
+            _load_calls()
+        if _cuda_call:
+            done = _cuda_call.exec(self._compiled[0] or self._compile(), inputs)
             if done is not None:
                 return done
+        import torch
         device = next((x.device for x in inputs if _on_cuda(x)), "cpu")
         return self._run_into_new(lambda shape: torch.empty(shape, dtype=torch.float32, device=device),
                                   inputs)
@@ -438,12 +447,16 @@ class Component:
         not ordered behind work that is still producing them.
         """
         program = self._compiled[0] or self._compile()
-        for kind in ("cuda", "host"):
-            native = _native.get(kind) or _native_call(kind)
-            if native is not None:
-                done = native.into(program, outputs, inputs)
-                if done is not None:
-                    return done
+        if _cuda_call is None or _host_call is None:
+            _load_calls()
+        if _cuda_call:
+            done = _cuda_call.into(program, outputs, inputs)
+            if done is not None:
+                return done
+        if _host_call:
+            done = _host_call.into(program, outputs, inputs)
+            if done is not None:
+                return done
         single = not isinstance(outputs, (tuple, list))
         if single:
             outputs = (outputs,)
