@@ -573,10 +573,12 @@ prepare_attention_mixed_kernel(PrepareMixedArgs a) {
 }
 
 // fp16 arm.  blockIdx.y = 0: K, one tile of 128 keys per block at a time: the tile is read once
-// twice (the second time from cache), its largest magnitude decides the power of two that brings it into
-// [2^14, 2^15), and fp16(K / that) is written with rows padded to d_pitch (pad columns zero).  An
-// outlier key therefore costs precision only to the 127 keys beside it.  blockIdx.y = 1: the fp16
-// V^T as in the mixed arm.
+// (twice, the second time from cache, without FEW_TILES), its largest magnitude decides the power of
+// two that brings it into [2^14, 2^15), and fp16(K / that) is written with rows padded to d_pitch (pad
+// columns zero).  An outlier key therefore costs precision only to the 127 keys beside it.
+// blockIdx.y = 1: the fp16 V^T as in the mixed arm.
+// Bound by HBM.  A thread's place in the tile comes from shifts: with a division of 64-bit numbers
+// by the row length per 16-byte load the K half of 64 heads x 2048 x 128 took 35 us for 100 MB, now 21.
 template <bool FEW_TILES>
 __global__ void __launch_bounds__(256)
 prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
@@ -588,7 +590,8 @@ prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
     prepare_v_f16(a, words, scratch);
     return;
   }
-  const size_t quads = a.d_pitch / 4;       // 4-column groups per (padded) key row, at most 32
+  // 4-column groups per (padded) key row: at most 32, rounded up to a power of two.
+  const unsigned across = 32 - __clz(static_cast<unsigned>(a.d_pitch / 4) - 1);
   const bool vec = (reinterpret_cast<uintptr_t>(a.k) & 15u) == 0;   // d is a multiple of 4
   // With few tiles (one head of a few thousand keys) the blocks are too few to hide two rounds of
   // loads each: a thread then keeps its share of the tile in registers (sixteen 16-byte loads in
@@ -601,20 +604,22 @@ prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
     const size_t keys = a.nk - key0 < 128 ? a.nk - key0 : 128;
     const float* src = a.k + (b * a.nk + key0) * a.d;
     __half* dst = a.k16 + (b * a.nk + key0) * a.d_pitch;
-    const size_t groups = keys * quads;
-    auto fetch = [&](size_t g) {
-      const size_t r = g / quads, c = (g - r * quads) * 4;
-      if (g >= groups || c >= a.d) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      const float* at = src + r * a.d + c;
+    // 2^across lanes take a row (at most 32, the rest of them idle past quads); a tile is
+    // 128 << across such places, at most 16 a thread.
+    const unsigned places = static_cast<unsigned>(keys) << across;
+    auto fetch = [&](unsigned g) {
+      const unsigned r = g >> across, c = (g & ((1u << across) - 1)) * 4;
+      if (g >= places || c >= a.d) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float* at = src + r * static_cast<unsigned>(a.d) + c;
       return vec ? *reinterpret_cast<const float4*>(at) : make_float4(at[0], at[1], at[2], at[3]);
     };
     // Pass 1: the tile's largest magnitude.  Pass 2 reads the same 64 KB again, from cache, unless
     // the thread's whole share (128 x 32 groups over 256 threads = 16) is still in registers.
     float m = 0.0f;
     float4 x[kBatch];
-    for (size_t g0 = threadIdx.x; g0 < groups; g0 += 256 * kBatch) {
+    for (unsigned g0 = threadIdx.x; g0 < places; g0 += 256 * kBatch) {
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) x[u] = fetch(g0 + static_cast<size_t>(u) * 256);
+      for (int u = 0; u < kBatch; ++u) x[u] = fetch(g0 + u * 256);
 #pragma unroll
       for (int u = 0; u < kBatch; ++u)
         m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
@@ -628,17 +633,17 @@ prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
     const float scale = f16_scale_for(all);
     const float inv = 1.0f / scale;
     if (threadIdx.x == 0) a.k_tile_scale[t] = scale;
-    for (size_t g0 = threadIdx.x; g0 < groups; g0 += 256 * kBatch) {
+    for (unsigned g0 = threadIdx.x; g0 < places; g0 += 256 * kBatch) {
       if (!FEW_TILES) {
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) x[u] = fetch(g0 + static_cast<size_t>(u) * 256);
+        for (int u = 0; u < kBatch; ++u) x[u] = fetch(g0 + u * 256);
       }
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const size_t g = g0 + static_cast<size_t>(u) * 256;
-        if (g < groups) {
-          const size_t r = g / quads, c = (g - r * quads) * 4;
-          *reinterpret_cast<uint2*>(dst + r * a.d_pitch + c) =
+        const unsigned g = g0 + u * 256;
+        const unsigned r = g >> across, c = (g & ((1u << across) - 1)) * 4;
+        if (g < places && c < a.d_pitch) {
+          *reinterpret_cast<uint2*>(dst + r * static_cast<unsigned>(a.d_pitch) + c) =
               pack4_f16(x[u].x * inv, x[u].y * inv, x[u].z * inv, x[u].w * inv);
         }
       }
