@@ -154,6 +154,8 @@ struct Shared {
   uint64_t m_ready[4];       // pipelined kernel: [tile & 3], the tile's reference maximum is published
 };
 
+constexpr int kSharedBytes = (static_cast<int>(sizeof(Shared)) + 63) / 64 * 64;
+
 // One contiguous run of key tiles of one row tile.
 struct Piece {
   int unit;        // row tile index over the whole call (head * q_tiles + tile)
@@ -342,6 +344,53 @@ __device__ __forceinline__ float stage_q_rows(const Params& p, Shared* sh, uint3
   return row_mul;
 }
 
+// A warp's exchange buffer of 32 rows x 16 columns: four 16-byte units a row, placed so that eight
+// lanes that read or write either two whole rows or one unit of eight rows meet no bank twice.
+constexpr int kSwapFloats = 32 * 16;
+__device__ __forceinline__ float4* swap_at(float* swap, int row, int unit) {
+  return reinterpret_cast<float4*>(swap + row * 16 + ((unit ^ ((row >> 1) & 3)) << 2));
+}
+
+// The last part of finish_piece for the pipelined kernel: this warp's 32 rows, columns [64h, 64h + 64)
+// of O, through the exchange buffer, so that a store writes 64 bytes of each of eight rows instead of
+// 16 of each of 32 (half sectors, and 32 lines to look up a store).
+__device__ __forceinline__ void store_o_rows(uint32_t o_tmem, float* dst0, long long rows, int dv, int h,
+                                             int dv_chunks, float inv, int lane, float* swap) {
+  const bool vec = dv % 4 == 0 && (reinterpret_cast<uintptr_t>(dst0) & 15u) == 0;
+#pragma unroll 1
+  for (int c = h * 2; c < h * 2 + 2 && c < dv_chunks; ++c) {
+    uint32_t o[32];
+    tmem_ld_32x32(o_tmem + c * 32, o);
+    tmem_wait_ld();
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e = part * 16 + u * 4;
+        *swap_at(swap, lane, u) = make_float4(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv,
+                                              __uint_as_float(o[e + 2]) * inv, __uint_as_float(o[e + 3]) * inv);
+      }
+      __syncwarp();
+      const int col = c * 32 + part * 16 + (lane & 3) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = i * 8 + (lane >> 2);
+        const float4 x = *swap_at(swap, row, lane & 3);
+        float* at = dst0 + static_cast<size_t>(row) * dv + col;
+        if (row < rows && vec && col < dv) {
+          *reinterpret_cast<float4*>(at) = x;
+        } else if (row < rows) {
+          if (col + 0 < dv) at[0] = x.x;
+          if (col + 1 < dv) at[1] = x.y;
+          if (col + 2 < dv) at[2] = x.z;
+          if (col + 3 < dv) at[3] = x.w;
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
 // End of a piece on the softmax warps: waits for the last P V, adds the two halves of the row
 // sum, normalises and stores this thread's columns [64h, 64h+64) of O (to the output, or to the
 // partial slot with its (m, l) when the piece covers only part of the keys).
@@ -349,7 +398,7 @@ __device__ __forceinline__ void finish_piece(const Params& p, Shared* sh, uint32
                                              int r, long long row, int b, bool whole, int part_slot,
                                              float l, float m_used, int dv_chunks,
                                              uint64_t* last_pv_done, uint32_t last_parity,
-                                             bool& dead) {
+                                             bool& dead, float* swap = nullptr) {
   if (!sh->give_up && !dead)
     dead = !mbar_wait_warp(last_pv_done, last_parity, &sh->abort, p.status, 209);
   sh->half_sum[h][r] = l;
@@ -369,6 +418,12 @@ __device__ __forceinline__ void finish_piece(const Params& p, Shared* sh, uint32
       p.part_m[prow] = m_used;
       p.part_l[prow] = l_total;
     }
+  }
+  if (swap) {
+    const int lane = r & 31;
+    store_o_rows(o_tmem, dst - static_cast<size_t>(lane) * p.dv, whole ? p.nq - (row - lane) : 32, p.dv, h,
+                 dv_chunks, inv, lane, swap);
+    return;
   }
   const bool vec_ok = (p.dv % 4 == 0) && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
   for (int c = h * 2; c < h * 2 + 2 && c < dv_chunks; ++c) {
@@ -935,6 +990,10 @@ __device__ __forceinline__ void named_sync(int id, int threads) {
 //   * Q of the next row block staged with one round of loads (each thread its own 64 columns, the
 //     two halves of a row's largest magnitude meeting through shared memory) instead of nine
 //     dependent rounds: 754 -> 829 TFLOP/s on one head of 16384, 972 -> 1015 on eight.
+//   * Q's loads and O's stores pass through an exchange buffer of 2 KB a warp (swap_at), four lanes a
+//     row: with a thread on a row of its own each instruction touched 32 lines and O was written in
+//     half sectors, ~8000 cycles a row tile: 64 heads x 2048 217 -> 178 us in this kernel, one head
+//     of 16384 162 -> 153.
 // setmaxnreg moves registers from the role and statistics warps to the softmax warps.
 //
 constexpr uint32_t kTmemP = 64;            // pipelined kernel: packed P, beside packed Q (0..63)
@@ -985,31 +1044,41 @@ __device__ __forceinline__ void setmaxnreg_inc() {
 // here too and only skips the work.
 template <Arm ARM>
 __device__ __forceinline__ float stage_q_half(const Params& p, Shared* sh, uint32_t tmem_q, int head,
-                                              int q_tile, int r, int h, int lane, int piece, bool idle) {
+                                              int q_tile, int r, int h, int lane, int piece, bool idle,
+                                              float* swap) {
   using G = Geometry<ARM>;
   float row_mul = kLog2E32;
-  const long long row = static_cast<long long>(q_tile) * kBQ + r;
-  const float* qrow = p.q + (static_cast<size_t>(head) * p.nq + row) * p.d;
-  const bool live = row < p.nq && !idle;
-  const bool vec = (reinterpret_cast<uintptr_t>(p.q) & 15u) == 0 && p.d % 4 == 0;
+  const long long row0 = static_cast<long long>(q_tile) * kBQ + (r - lane);   // of this warp's 32
+  const float* q0 = p.q + (static_cast<size_t>(head) * p.nq + row0) * p.d;
+  const bool vec = (reinterpret_cast<uintptr_t>(p.q) & 15u) == 0;
   float qs = 1.0f;                             // a scale on the logits is a scale on Q
   if (p.logit_scale) {
     qs = __ldg(p.logit_scale);
     if (p.logit_divide) qs = 1.0f / qs;
   }
+  // Four lanes take 16 columns of a row, a load eight rows; the warp's exchange then gives every
+  // thread the row it owns (each thread loading its own row is 32 lines a load).
   float4 x[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) {
-    const int col = h * 64 + 4 * e;
+    const int at = (e & 3) * 8 + (lane >> 2), col = h * 64 + (e >> 2) * 16 + (lane & 3) * 4;
+    const float* from = q0 + static_cast<size_t>(at) * p.d + col;
+    const bool live = row0 + at < p.nq && col < p.d && !idle;      // d is a multiple of four
     x[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (live && vec && col + 4 <= p.d) {
-      x[e] = *reinterpret_cast<const float4*>(qrow + col);
+    if (live && vec) {
+      x[e] = *reinterpret_cast<const float4*>(from);
     } else if (live) {
-      if (col + 0 < p.d) x[e].x = qrow[col + 0];
-      if (col + 1 < p.d) x[e].y = qrow[col + 1];
-      if (col + 2 < p.d) x[e].z = qrow[col + 2];
-      if (col + 3 < p.d) x[e].w = qrow[col + 3];
+      x[e] = make_float4(from[0], from[1], from[2], from[3]);
     }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) *swap_at(swap, e * 8 + (lane >> 2), lane & 3) = x[4 * c + e];
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[4 * c + e] = *swap_at(swap, lane, e);
+    __syncwarp();
   }
 #pragma unroll
   for (int e = 0; e < 16; ++e) { x[e].x *= qs; x[e].y *= qs; x[e].z *= qs; x[e].w *= qs; }
@@ -1392,6 +1461,7 @@ attention_pipelined_kernel(const __grid_constant__ CUtensorMap map_k,
     const uint32_t p_tmem = tmem_base + lane_bits + kTmemP;
     const uint32_t tmem_q = tmem_base + lane_bits + kTmemQ;
     const int dv_chunks = (p.dv + 31) / 32;
+    float* swap = reinterpret_cast<float*>(ring + kRingBytes + kSharedBytes) + (warp - 8) * kSwapFloats;
     int it = 0;                               // key tiles of the pieces before this one
     long long wait_s = 0, c_a = 0, c_b = 0, c_exp = 0, c_tail = 0;   // kProf: cycles per phase
     const long long t_start = tick<kProf>();
@@ -1415,7 +1485,7 @@ attention_pipelined_kernel(const __grid_constant__ CUtensorMap map_k,
       const bool whole = pc.whole;
       const int part_slot = 2 * static_cast<int>(blockIdx.x) + pc.ordinal;
 
-      if (piece == 0) row_mul = stage_q_half<ARM>(p, sh, tmem_q, b, qt, r, h, lane, 0, false);
+      if (piece == 0) row_mul = stage_q_half<ARM>(p, sh, tmem_q, b, qt, r, h, lane, 0, false, swap);
 
       // The piece after this one, whose Q is staged at the end of this one.
       float next_row_mul = kLog2E32;
@@ -1569,10 +1639,11 @@ attention_pipelined_kernel(const __grid_constant__ CUtensorMap map_k,
       // Q of the next piece, before this one's epilogue, so that the Q K^T issuer can run the next
       // piece's first tiles while O is being read out below.  (The warpgroup that owns the last
       // tile has seen its S; the other one waited for it above.)
-      if (has_next) next_row_mul = stage_q_half<ARM>(p, sh, tmem_q, next_b, next_qt, r, h, lane, piece + 1, dead);
+      if (has_next)
+        next_row_mul = stage_q_half<ARM>(p, sh, tmem_q, next_b, next_qt, r, h, lane, piece + 1, dead, swap);
 
       finish_piece(p, sh, o_tmem, h, r, row, b, whole, part_slot, l, m_final, dv_chunks,
-                   &sh->pv_done[last & 3], static_cast<uint32_t>((last >> 2) & 1), dead);
+                   &sh->pv_done[last & 3], static_cast<uint32_t>((last >> 2) & 1), dead, swap);
       if (sh->give_up) break;
       tc_fence_before_sync();
       __syncwarp();
@@ -1799,7 +1870,8 @@ int attention_tcgen05(const float* q, const void* k, const void* vt, float* o, s
     return fail("ib_attention: shape too large");
   if (d % 4 != 0 || d < 4 || d > 128 || dv < 1 || dv > 128)
     return fail("ib_attention: head dimensions outside the fused kernel's range");
-  const int smem_bytes = 1024 + kRingBytes + static_cast<int>(sizeof(Shared)) + 64;
+  const int smem_bytes = 1024 + kRingBytes + kSharedBytes + 8 * kSwapFloats * static_cast<int>(sizeof(float));
+  static_assert(1024 + kRingBytes + kSharedBytes + 8 * kSwapFloats * sizeof(float) <= 232448, "shared memory of a CTA");
   // The opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of each kernel.
   {
     static OncePerDevice configured;
@@ -1914,8 +1986,9 @@ int attention_tcgen05(const float* q, const void* k, const void* vt, float* o, s
   if (launched != cudaSuccess)
     return fail(std::string("ib_attention (tcgen05): launch failed: ") + cudaGetErrorString(launched));
   count_launch();
-  // Tail row tiles shared by several CTA ranges exist unless the ranges fall on tile boundaries.
-  if (tail_units > 0 && !(p.iters_rem == 0 && p.iters_base % p.kv_coarse == 0)) {
+  // Tail row tiles shared by several CTA ranges exist unless the ranges fall on tile boundaries (always
+  // so where a row tile is one granule: 64 heads x 2048, 3 us of a kernel that found nothing to do).
+  if (tail_units > 0 && p.kv_coarse > 1 && !(p.iters_rem == 0 && p.iters_base % p.kv_coarse == 0)) {
     CombineArgs a{p.part_o, p.part_m, p.part_l, o, p.nq, p.dv, p.q_tiles, p.kv_coarse, ctas,
                   p.full_waves * ctas, p.iters_base, p.iters_rem};
     cfg.numAttrs = g_dependent_launch ? 1 : 0;

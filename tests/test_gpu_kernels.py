@@ -685,6 +685,29 @@ def test_attention_tf32_f16_shapes(lib, oracle, torch, nq, nk, d, dv, precision)
     assert max_rel_to_peak(got, oracle.attention_fused(q, k, v)) <= TOL_TF32
 
 
+@pytest.mark.parametrize("precision,tol", [(F16, TOL_TF32), (BF16, TOL_BF16)])
+@pytest.mark.parametrize("nq,nk,d,dv,shift", [(1030, 200, 84, 50, 0), (1030, 130, 128, 100, 0), (1000, 129, 20, 128, 1)])
+def test_attention_16_bit_row_tiles_in_turn(lib, torch, precision, tol, nq, nk, d, dv, shift):
+    # More row tiles than SMs, so that Q of a row tile is loaded and O stored between others; rows,
+    # features and columns that end inside a warp's exchange, and Q and O off 16-byte boundaries.
+    batch = 20
+    q = torch.randn(batch * nq * d + shift, device="cuda")[shift:] * d ** -0.5
+    k, v = torch.randn(batch, nk, d, device="cuda"), torch.randn(batch, nk, dv, device="cuda")
+    if shift:
+        q = torch.cat([q.new_zeros(shift), q])[shift:]
+    o = torch.full((batch * nq * dv + shift + 4,), float("nan"), device="cuda")
+    ws_bytes = lib.ib_attention_workspace_bytes(batch, nq, nk, d, dv, 0, precision)
+    ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device="cuda")
+    ok(lib, lib.ib_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), o[shift:].data_ptr(), batch, nq, nk, d, dv,
+                             0, precision, 0, ws.data_ptr(), ws_bytes, None))
+    torch.cuda.synchronize()
+    q3 = q.reshape(batch, nq, d).double()
+    want = torch.softmax(q3 @ k.double().transpose(1, 2), -1) @ v.double()
+    got = o[shift:shift + batch * nq * dv].reshape(batch, nq, dv).double()
+    assert ((got - want).abs().max() / want.abs().max()).item() <= tol
+    assert torch.isnan(o[:shift]).all() and torch.isnan(o[shift + batch * nq * dv:]).all()
+
+
 def test_attention_f16_is_as_accurate_as_tf32(lib, oracle, torch):
     # fp16 operands carry TF32's 10-bit mantissa: against an exact reference the fp16 arm's error
     # must sit where the TF32 arm's does, not where bf16's (8 bits) does.
