@@ -344,13 +344,6 @@ __device__ __forceinline__ float stage_q_rows(const Params& p, Shared* sh, uint3
   return row_mul;
 }
 
-// A warp's exchange buffer of 32 rows x 16 columns: four 16-byte units a row, placed so that eight
-// lanes that read or write either two whole rows or one unit of eight rows meet no bank twice.
-constexpr int kSwapFloats = 32 * 16;
-__device__ __forceinline__ float4* swap_at(float* swap, int row, int unit) {
-  return reinterpret_cast<float4*>(swap + row * 16 + ((unit ^ ((row >> 1) & 3)) << 2));
-}
-
 // The last part of finish_piece for the pipelined kernel: this warp's 32 rows, columns [64h, 64h + 64)
 // of O, through the exchange buffer, so that a store writes 64 bytes of each of eight rows instead of
 // 16 of each of 32 (half sectors, and 32 lines to look up a store).
@@ -1841,6 +1834,7 @@ int device_sms() {
 
 }  // namespace
 
+bool dependent_launch() { return g_dependent_launch; }
 void set_attention_profile(unsigned long long* p) { g_attention_profile = p; }
 void set_reserved_sms(int n) { g_reserved_sms.store(n < 0 ? 0 : n); }
 int reserved_sms() { return g_reserved_sms.load(); }

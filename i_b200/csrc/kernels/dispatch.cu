@@ -236,21 +236,15 @@ extern "C" size_t ib_contract_workspace_bytes(size_t batch, size_t m, size_t n, 
   if (!wants_tensor(precision, flop)) return fp32_bytes;
   if (precision == IB_PRECISION_AUTO && contract_prefers_f16(m, n, k)) precision = IB_PRECISION_F16;
   if (precision == IB_PRECISION_F16) {
-    // fp16 copies of both operands plus one scale per row; fp32 transposes first when needed.
+    // fp16 copies of both operands plus one scale per row.
     const size_t kp = round_up(k, 8);
-    size_t bytes = carve_bytes((batch * m * kp + 1) / 2) + carve_bytes((batch * n * kp + 1) / 2) +
-                   carve_bytes(batch * m) + carve_bytes(batch * n);
-    if (!a_kmajor) bytes += carve_bytes(batch * m * k);
-    if (!b_kmajor) bytes += carve_bytes(batch * n * k);
-    return bytes;
+    return carve_bytes((batch * m * kp + 1) / 2) + carve_bytes((batch * n * kp + 1) / 2) + carve_bytes(batch * m) +
+           carve_bytes(batch * n);
   }
   if (precision == IB_PRECISION_BF16) {
-    // bf16 copies of both operands ([rows][k rounded up to 8]); fp32 transposes first when needed.
+    // bf16 copies of both operands ([rows][k rounded up to 8]).
     const size_t kp = round_up(k, 8);
-    size_t bytes = carve_bytes((batch * m * kp + 1) / 2) + carve_bytes((batch * n * kp + 1) / 2);
-    if (!a_kmajor) bytes += carve_bytes(batch * m * k);
-    if (!b_kmajor) bytes += carve_bytes(batch * n * k);
-    return bytes;
+    return carve_bytes((batch * m * kp + 1) / 2) + carve_bytes((batch * n * kp + 1) / 2);
   }
   if (!contract_shape_ok(k)) return fp32_bytes;
   // Copies of the result when the k range is cut into parts.
@@ -465,22 +459,9 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
     float* a_scale = ws.take(batch * m);
     float* b_scale = ws.take(batch * n);
     if (!a16 || !b16 || !a_scale || !b_scale) return fail(small);
-    const float* ak = a;
-    const float* bk = b;
-    if (!a_kmajor) {
-      float* t = ws.take(batch * m * k);
-      if (!t) return fail(small);
-      if (int rc = transpose_batched(a, t, batch, k, m, k, false, s)) return rc;
-      ak = t;
-    }
-    if (!b_kmajor) {
-      float* t = ws.take(batch * n * k);
-      if (!t) return fail(small);
-      if (int rc = transpose_batched(b, t, batch, k, n, k, false, s)) return rc;
-      bk = t;
-    }
-    if (int rc = convert_f16_rows_scaled(ak, a16, a_scale, batch * m, k, kp, s)) return rc;
-    if (int rc = convert_f16_rows_scaled(bk, b16, b_scale, batch * n, k, kp, s)) return rc;
+    if (int rc = prepare_contract_operands(a, a_kmajor != 0, a16, a_scale, b, b_kmajor != 0, b16, b_scale, batch, m,
+                                           n, k, kp, s))
+      return rc;
     return gemm_tcgen05_f16(a16, b16, a_scale, b_scale, c, batch, m, n, k, kp, s, geometry, fused);
   }
   if (precision == IB_PRECISION_BF16) {
@@ -492,22 +473,9 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
     float* a16 = ws.take((batch * m * kp + 1) / 2);
     float* b16 = ws.take((batch * n * kp + 1) / 2);
     if (!a16 || !b16) return fail(small);
-    const float* ak = a;
-    const float* bk = b;
-    if (!a_kmajor) {
-      float* t = ws.take(batch * m * k);
-      if (!t) return fail(small);
-      if (int rc = transpose_batched(a, t, batch, k, m, k, false, s)) return rc;
-      ak = t;
-    }
-    if (!b_kmajor) {
-      float* t = ws.take(batch * n * k);
-      if (!t) return fail(small);
-      if (int rc = transpose_batched(b, t, batch, k, n, k, false, s)) return rc;
-      bk = t;
-    }
-    if (int rc = convert_bf16_rows(ak, a16, batch * m, k, kp, s)) return rc;
-    if (int rc = convert_bf16_rows(bk, b16, batch * n, k, kp, s)) return rc;
+    if (int rc = prepare_contract_operands(a, a_kmajor != 0, a16, nullptr, b, b_kmajor != 0, b16, nullptr, batch, m,
+                                           n, k, kp, s))
+      return rc;
     return gemm_tcgen05_bf16(a16, b16, c, batch, m, n, k, kp, s, geometry, fused);
   }
   if (wants_tensor(precision, flop) && contract_shape_ok(k)) {

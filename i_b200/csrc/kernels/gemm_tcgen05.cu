@@ -32,6 +32,7 @@ using namespace sm100;
 constexpr int kBM = 128;
 constexpr int kBK = 32;            // fp32 per 128-byte swizzled row
 constexpr int kStages = 4;
+constexpr int kSwapBytes = 4 * kSwapFloats * 4;    // an exchange buffer per epilogue warp
 constexpr int kGroupN = 12;        // n-tiles per raster group unless the caller's geometry says otherwise
 constexpr int kThreads = 192;
 
@@ -41,7 +42,7 @@ struct Smem {
   static constexpr int kBBytes = BN * kBK * 4;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarrierBytes = 256;
-  static constexpr int kTotal = kStages * kStageBytes + kBarrierBytes + 1024;  // + alignment slack
+  static constexpr int kTotal = kStages * kStageBytes + kBarrierBytes + kSwapBytes + 1024;  // + alignment slack
 };
 
 struct TileCoord {
@@ -66,13 +67,61 @@ __device__ __forceinline__ TileCoord tile_coord(long long id, int tiles_m, int t
   return t;
 }
 
-// The pointwise operators of a GemmEpilogue over the 32 consecutive columns of one row a thread
-// holds.  `grow` is the row over all batch entries.  Every operator sits behind a warp-uniform
-// switch inside a loop that is not unrolled, so its operands are materialised values: nothing is
-// contracted into a multiply-add across operators, and the result has the bits the separate
-// pointwise kernels give.
-__device__ __forceinline__ void apply_epilogue(const GemmEpilogue& e, uint32_t (&r)[32], size_t grow,
-                                               int col0, int n, bool vec_ok) {
+// What the epilogue warps do with 32 columns of their 32 rows.  The accumulator arrives with a row per
+// thread; the warp's exchange buffer turns that into four lanes a row, so that operands and results move
+// in 64-byte pieces of eight rows an instruction (a thread on its own row met 32 lines an instruction and
+// wrote half sectors: 8192 x 8192 x 4096 on fp16 operands 414 -> 369 us in this kernel, its stores
+// having competed with the operand loads).  Value v = part * 16 + i * 4 + j of a thread is then row
+// i * 8 + lane / 4 and column col0 + part * 16 + (lane % 4) * 4 + j.
+struct EpilogueRows {
+  float* c;              // the warp's first row
+  size_t grow;           // its number over all batch entries
+  int rows;              // rows of the result from there on
+  int n;
+  bool vec;              // n and c allow 16-byte accesses
+  const float* rs;       // row scales from the first row on, or null
+  const float* cs;       // column scales of the batch entry, or null
+};
+
+__device__ __forceinline__ void load_columns(float (&t)[4], const float* p, int col, int n, bool vec) {
+  if (vec && col < n && (reinterpret_cast<uintptr_t>(p + col) & 15u) == 0) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(p + col));
+    t[0] = x.x; t[1] = x.y; t[2] = x.z; t[3] = x.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[j] = col + j < n ? __ldg(p + col + j) : 0.0f;
+  }
+}
+
+// What 32 columns need besides the accumulator, asked for before it: the column scales, and the first
+// operand that has one value per column (a bias).  Asked for after the exchange instead, each of a tile's
+// eight steps waited for L2, exposed where a result is a wave or two of tiles.
+struct ColumnsAhead {
+  float scale[2][4];
+  float operand[2][4];
+};
+
+__device__ __forceinline__ int first_per_column(const GemmEpilogue& e) {
+  for (int k = 0; k < e.n_ops; ++k)
+    if (e.which[k] >= 0 && e.mode[e.which[k]] == 2) return k;
+  return -1;
+}
+
+__device__ __forceinline__ void look_ahead(ColumnsAhead& x, const GemmEpilogue& e, const EpilogueRows& at, int col0,
+                                           int per_column) {
+  const int col = col0 + (threadIdx.x & 3) * 4;
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    if (at.cs) load_columns(x.scale[part], at.cs, col + part * 16, at.n, at.vec);
+    if (per_column >= 0) load_columns(x.operand[part], e.operand[e.which[per_column]], col + part * 16, at.n, at.vec);
+  }
+}
+
+// The pointwise operators of a GemmEpilogue.  Every operator sits behind a warp-uniform switch inside a
+// loop that is not unrolled, so its operands are materialised values: nothing is contracted into a
+// multiply-add across operators, and the result has the bits the separate pointwise kernels give.
+__device__ __forceinline__ void apply_epilogue(const GemmEpilogue& e, float (&r)[32], const EpilogueRows& at,
+                                               int row0, int col, const ColumnsAhead& ahead, int per_column) {
 #pragma unroll 1
   for (int k = 0; k < e.n_ops; ++k) {
     float t[32];
@@ -80,24 +129,30 @@ __device__ __forceinline__ void apply_epilogue(const GemmEpilogue& e, uint32_t (
     if (w >= 0) {
       const float* p = e.operand[w];
       const int mode = e.mode[w];
-      if (mode == 1 || mode == 3) {
-        const float s = __ldg(mode == 1 ? p + grow : p);
+      if (mode == 0) {
 #pragma unroll
-        for (int v = 0; v < 32; ++v) t[v] = s;
+        for (int v = 0; v < 8; ++v) {
+          const int row = row0 + (v & 3) * 8, c = col + (v >> 2) * 16;
+          float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          if (row < at.rows) load_columns(x, p + (at.grow + row) * static_cast<size_t>(at.n), c, at.n, at.vec);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) t[4 * v + j] = x[j];
+        }
+      } else if (k == per_column) {
+#pragma unroll
+        for (int v = 0; v < 32; ++v) t[v] = ahead.operand[v >> 4][v & 3];
+      } else if (mode == 2) {
+        float x[2][4];
+        load_columns(x[0], p, col, at.n, at.vec);
+        load_columns(x[1], p, col + 16, at.n, at.vec);
+#pragma unroll
+        for (int v = 0; v < 32; ++v) t[v] = x[v >> 4][v & 3];
       } else {
-        const float* src = mode == 0 ? p + grow * static_cast<size_t>(n) + col0 : p + col0;
-        if (vec_ok && col0 + 32 <= n && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
 #pragma unroll
-          for (int v = 0; v < 8; ++v) {
-            const float4 x = __ldg(reinterpret_cast<const float4*>(src) + v);
-            t[4 * v + 0] = x.x;
-            t[4 * v + 1] = x.y;
-            t[4 * v + 2] = x.z;
-            t[4 * v + 3] = x.w;
-          }
-        } else {
+        for (int i = 0; i < 4; ++i) {
+          const float x = mode == 3 ? __ldg(p) : row0 + i * 8 < at.rows ? __ldg(p + at.grow + row0 + i * 8) : 0.0f;
 #pragma unroll
-          for (int v = 0; v < 32; ++v) t[v] = col0 + v < n ? __ldg(src + v) : 0.0f;
+          for (int j = 0; j < 4; ++j) t[4 * i + j] = t[16 + 4 * i + j] = x;
         }
       }
     }
@@ -105,14 +160,11 @@ __device__ __forceinline__ void apply_epilogue(const GemmEpilogue& e, uint32_t (
 #define IB_EPILOGUE_CASE(OP)                                                                   \
   case OP:                                                                                     \
     if (w < 0) {                                                                               \
-      _Pragma("unroll") for (int v = 0; v < 32; ++v)                                           \
-          r[v] = __float_as_uint(apply_unary(OP, __uint_as_float(r[v])));                      \
+      _Pragma("unroll") for (int v = 0; v < 32; ++v) r[v] = apply_unary(OP, r[v]);             \
     } else if (right) {                                                                        \
-      _Pragma("unroll") for (int v = 0; v < 32; ++v)                                           \
-          r[v] = __float_as_uint(apply_binary(OP, t[v], __uint_as_float(r[v])));               \
+      _Pragma("unroll") for (int v = 0; v < 32; ++v) r[v] = apply_binary(OP, t[v], r[v]);      \
     } else {                                                                                   \
-      _Pragma("unroll") for (int v = 0; v < 32; ++v)                                           \
-          r[v] = __float_as_uint(apply_binary(OP, __uint_as_float(r[v]), t[v]));               \
+      _Pragma("unroll") for (int v = 0; v < 32; ++v) r[v] = apply_binary(OP, r[v], t[v]);      \
     }                                                                                          \
     break;
     switch (e.op[k]) {
@@ -126,41 +178,46 @@ __device__ __forceinline__ void apply_epilogue(const GemmEpilogue& e, uint32_t (
   }
 }
 
-// What an epilogue thread does with 32 consecutive columns of its row: the scales of the fp16
-// arm (C[i][j] = acc * row_scale[i] * col_scale[j], exact: powers of two), the caller's pointwise
-// operators, the store.
-__device__ __forceinline__ void finish_columns(uint32_t (&r)[32], float* crow, size_t grow, bool row_ok,
-                                               float rs, const float* cs, int col0, int n, bool vec_ok,
-                                               const GemmEpilogue& e) {
-  if (!row_ok) return;
-  if (cs) {
-    if (vec_ok && col0 + 32 <= n && (reinterpret_cast<uintptr_t>(cs) & 15u) == 0) {
+// The scales of the fp16 arm (C[i][j] = acc * row_scale[i] * col_scale[j], exact: powers of two), the
+// caller's pointwise operators, the store.
+__device__ __forceinline__ void finish_columns(const uint32_t (&acc)[32], const EpilogueRows& at, int col0,
+                                               const GemmEpilogue& e, const float (&rs)[4],
+                                               const ColumnsAhead& ahead, int per_column, float* swap) {
+  const int lane = threadIdx.x & 31, row0 = lane >> 2, col = col0 + (lane & 3) * 4;
+  float r[32];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const float4 w = __ldg(reinterpret_cast<const float4*>(cs + col0) + v);
-        r[4 * v + 0] = __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[4 * v + 0]), rs), w.x));
-        r[4 * v + 1] = __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[4 * v + 1]), rs), w.y));
-        r[4 * v + 2] = __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[4 * v + 2]), rs), w.z));
-        r[4 * v + 3] = __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[4 * v + 3]), rs), w.w));
-      }
-    } else {
+  for (int part = 0; part < 2; ++part) {
+    __syncwarp();
 #pragma unroll
-      for (int v = 0; v < 32; ++v)
-        if (col0 + v < n)
-          r[v] = __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[v]), rs), __ldg(cs + col0 + v)));
+    for (int u = 0; u < 4; ++u) {
+      const int v = part * 16 + u * 4;
+      *swap_at(swap, lane, u) = make_float4(__uint_as_float(acc[v]), __uint_as_float(acc[v + 1]),
+                                            __uint_as_float(acc[v + 2]), __uint_as_float(acc[v + 3]));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 x = *swap_at(swap, i * 8 + row0, lane & 3);
+      r[part * 16 + i * 4] = x.x; r[part * 16 + i * 4 + 1] = x.y;
+      r[part * 16 + i * 4 + 2] = x.z; r[part * 16 + i * 4 + 3] = x.w;
     }
   }
-  if (e.n_ops) apply_epilogue(e, r, grow, col0, n, vec_ok);
-  if (vec_ok && col0 + 32 <= n) {
+  if (at.cs) {
 #pragma unroll
-    for (int v = 0; v < 8; ++v)
-      *reinterpret_cast<float4*>(crow + col0 + 4 * v) =
-          make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                      __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-  } else {
+    for (int v = 0; v < 32; ++v) r[v] = __fmul_rn(__fmul_rn(r[v], rs[(v >> 2) & 3]), ahead.scale[v >> 4][v & 3]);
+  }
+  if (e.n_ops) apply_epilogue(e, r, at, row0, col, ahead, per_column);
 #pragma unroll
-    for (int v = 0; v < 32; ++v)
-      if (col0 + v < n) crow[col0 + v] = __uint_as_float(r[v]);
+  for (int v = 0; v < 8; ++v) {
+    const int row = row0 + (v & 3) * 8, c = col + (v >> 2) * 16;
+    float* to = at.c + static_cast<size_t>(row) * at.n + c;
+    if (row < at.rows && at.vec && c < at.n) {
+      *reinterpret_cast<float4*>(to) = make_float4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+    } else if (row < at.rows) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < at.n) to[j] = r[4 * v + j];
+    }
   }
 }
 
@@ -218,6 +275,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (lane == 0) {
       tma_prefetch_descriptor(&map_a);
       tma_prefetch_descriptor(&map_b);
+      grid_dependency_wait();                // the operands may come from the kernel before this one
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -282,28 +340,34 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    float* swap = reinterpret_cast<float*>(smem + kStages * L::kStageBytes + L::kBarrierBytes) + (warp - 2) * kSwapFloats;
+    grid_dependency_wait();                  // the scales come from the conversion before this kernel
+    const int per_column = first_per_column(epilogue);
     const bool vec_ok = (n % 4 == 0) && ((reinterpret_cast<uintptr_t>(c) & 15u) == 0);
     for (long long id = blockIdx.x; ok && id < total_tiles; id += gridDim.x) {
       const TileCoord t = tile_coord(id, tiles_m, tiles_n, group_n);
+      const int row = t.m_tile * kBM + quad * 32;
+      const size_t grow = static_cast<size_t>(t.batch) * m + row;
+      const EpilogueRows at{c + grow * n, grow, m - row, n, vec_ok, row_scale ? row_scale + grow : nullptr,
+                            col_scale ? col_scale + static_cast<size_t>(t.batch) * n : nullptr};
+      float rs[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        rs[i] = row_scale && (lane >> 2) + i * 8 < at.rows ? __ldg(at.rs + (lane >> 2) + i * 8) : 1.0f;
       ok = mbar_wait(&acc_full[acc], acc_phase, abort, status, 104);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
-      const int row = t.m_tile * kBM + quad * 32 + lane;
-      float* crow = c + (static_cast<size_t>(t.batch) * m + row) * n;
-      // fp16 operands stored over powers of two: C[i][j] = acc * row_scale[i] * col_scale[j], exact.
-      const float rs = row_scale && row < m ? row_scale[static_cast<size_t>(t.batch) * m + row] : 1.0f;
-      const float* cs = col_scale ? col_scale + static_cast<size_t>(t.batch) * n : nullptr;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
                              static_cast<uint32_t>(acc * BN);
 #pragma unroll 1
       for (int chunk = 0; chunk < BN / 32; ++chunk) {
         uint32_t r[32];
+        ColumnsAhead ahead;
+        look_ahead(ahead, epilogue, at, t.n_tile * BN + chunk * 32, per_column);
         tmem_ld_32x32(taddr + chunk * 32, r);
         tmem_wait_ld();
-        const int col0 = t.n_tile * BN + chunk * 32;
-        finish_columns(r, crow, static_cast<size_t>(t.batch) * m + row, row < m, rs, cs, col0, n, vec_ok,
-                       epilogue);
+        finish_columns(r, at, t.n_tile * BN + chunk * 32, epilogue, rs, ahead, per_column, swap);
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -353,7 +417,7 @@ __device__ long long g_pair_prof[16];
 #endif
 constexpr int kPairStages = 6;
 constexpr int kPairStageBytes = 2 * kBM * kBK * 4;      // A box + B box, 16 KB each
-constexpr int kPairSmem = kPairStages * kPairStageBytes + 512 + 1024;
+constexpr int kPairSmem = kPairStages * kPairStageBytes + 512 + kSwapBytes + 1024;
 
 template <Kind KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
@@ -412,6 +476,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (lane == 0) {
       tma_prefetch_descriptor(&map_a);
       tma_prefetch_descriptor(&map_b);
+      grid_dependency_wait();                // the operands may come from the kernel before this one
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -516,27 +581,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    float* swap = reinterpret_cast<float*>(smem + kPairStages * kPairStageBytes + 512) + (warp - 2) * kSwapFloats;
+    grid_dependency_wait();                  // the scales come from the conversion before this kernel
+    const int per_column = first_per_column(epilogue);
     const bool vec_ok = (n % 4 == 0) && ((reinterpret_cast<uintptr_t>(c) & 15u) == 0);
     for (long long id = pair; ok && id < total_tiles; id += pairs) {
       const TileCoord t = tile_coord(id, tiles_m, tiles_n, group_n);
+      const int row = t.m_tile * 2 * kBM + static_cast<int>(rank) * kBM + quad * 32;
+      const size_t grow = static_cast<size_t>(t.batch) * m + row;
+      const EpilogueRows at{c + grow * n, grow, m - row, n, vec_ok, row_scale ? row_scale + grow : nullptr,
+                            col_scale ? col_scale + static_cast<size_t>(t.batch) * n : nullptr};
+      float rs[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        rs[i] = row_scale && (lane >> 2) + i * 8 < at.rows ? __ldg(at.rs + (lane >> 2) + i * 8) : 1.0f;
       ok = mbar_wait_cluster(&acc_full[acc], acc_phase, abort, status, 116);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
-      const int row = t.m_tile * 2 * kBM + static_cast<int>(rank) * kBM + quad * 32 + lane;
-      float* crow = c + (static_cast<size_t>(t.batch) * m + row) * n;
-      const float rs = row_scale && row < m ? row_scale[static_cast<size_t>(t.batch) * m + row] : 1.0f;
-      const float* cs = col_scale ? col_scale + static_cast<size_t>(t.batch) * n : nullptr;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
                              static_cast<uint32_t>(acc * BN);
 #pragma unroll 1
       for (int chunk = 0; chunk < BN / 32; ++chunk) {
         uint32_t r[32];
+        ColumnsAhead ahead;
+        look_ahead(ahead, epilogue, at, t.n_tile * BN + chunk * 32, per_column);
         tmem_ld_32x32(taddr + chunk * 32, r);
         tmem_wait_ld();
-        const int col0 = t.n_tile * BN + chunk * 32;
-        finish_columns(r, crow, static_cast<size_t>(t.batch) * m + row, row < m, rs, cs, col0, n, vec_ok,
-                       epilogue);
+        finish_columns(r, at, t.n_tile * BN + chunk * 32, epilogue, rs, ahead, per_column, swap);
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -554,6 +626,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     tc_fence_after_sync();
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }
+}
+
+// The 16-bit kernels follow the conversion of their operands: launched so that their set-up runs under
+// its tail (they wait for it before the first read; everything older it has waited for itself).
+template <class... Params, class... Args>
+int launch_after_conversion(void (*kernel)(Params...), unsigned grid, int smem_bytes, cudaStream_t s, bool converted,
+                            Args... args) {
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+  cfg.stream = s;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = converted && dependent_launch() ? 1 : 0;
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (rc != cudaSuccess) return fail(std::string("ib_contract (tcgen05): launch failed: ") + cudaGetErrorString(rc));
+  count_launch();
+  return 0;
 }
 
 template <Kind KIND>
@@ -579,11 +672,10 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, float* c, si
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t pairs = std::min(tiles, static_cast<size_t>(sms / 2));
-  gemm_pair_kernel<KIND><<<static_cast<unsigned>(2 * pairs), kThreads, kPairSmem, s>>>(
-      map_a, map_b, c, static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
+  return launch_after_conversion(
+      gemm_pair_kernel<KIND>, static_cast<unsigned>(2 * pairs), kPairSmem, s, KIND == Kind::BF16, map_a, map_b, c, static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
       static_cast<int>(batch), status, row_scale, col_scale, f16_operands ? 1 : 0,
       group_n > 0 ? group_n : kGroupN, e ? *e : GemmEpilogue{});
-  return check_launch("ib_contract (tcgen05 pair)");
 }
 
 template <int BN, Kind KIND>
@@ -612,11 +704,10 @@ int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, float* c, size_t 
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = static_cast<int>(tiles < static_cast<size_t>(sms) ? tiles : sms);
-  gemm_tf32_kernel<BN, KIND><<<grid, kThreads, Smem<BN>::kTotal, s>>>(
-      map_a, map_b, c, static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
+  return launch_after_conversion(
+      gemm_tf32_kernel<BN, KIND>, static_cast<unsigned>(grid), Smem<BN>::kTotal, s, KIND == Kind::BF16, map_a, map_b, c, static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
       static_cast<int>(batch), status, row_scale, col_scale, f16_operands ? 1 : 0,
       group_n > 0 ? group_n : kGroupN, e ? *e : GemmEpilogue{});
-  return check_launch("ib_contract (tcgen05 tf32)");
 }
 
 }  // namespace

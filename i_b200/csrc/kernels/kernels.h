@@ -111,14 +111,19 @@ int gemm_tcgen05_f16(const void* a16, const void* b16, const float* a_scale, con
 int gemm_tcgen05_bf16(const void* a16, const void* b16, float* c, size_t batch, size_t m, size_t n,
                       size_t k, size_t k_pitch, cudaStream_t s, GemmGeometry g = {},
                       const GemmEpilogue* e = nullptr);
+// Both operands of a contraction for the 16-bit arms, in one launch: [batch][rows][kp] with kp = k
+// rounded up to 8, pad zero, from [rows][k] (kmajor) or [k][rows].  With scales fp16(x / scale[row]), the
+// row's largest magnitude brought into [2^14, 2^15); without (both null) bf16.
+int prepare_contract_operands(const float* a, bool a_kmajor, void* a16, float* a_scale, const float* b,
+                              bool b_kmajor, void* b16, float* b_scale, size_t batch, size_t m, size_t n,
+                              size_t k, size_t kp, cudaStream_t s);
 // out[r][c] = bf16(in[r][c]) (round to nearest even) for a [rows][cols] fp32 array; `out_pitch` in
 // elements, columns cols..out_pitch-1 are zeroed.
-// fp16 rows over one power of two each: out[r][c] = fp16(in[r][c] / scale[r]), scale[r] bringing the
-// row's largest magnitude into [2^14, 2^15); out_pitch % 8 == 0, pad columns zero.
-int convert_f16_rows_scaled(const float* in, void* out, float* scale, size_t rows, size_t cols,
-                            size_t out_pitch, cudaStream_t s);
 int convert_bf16_rows(const float* in, void* out, size_t rows, size_t cols, size_t out_pitch,
                       cudaStream_t s);
+
+// Whether a call's kernels may be launched under the tail of the one before (I_B200_DEPENDENT_LAUNCH).
+bool dependent_launch();
 
 // attention_tcgen05.cu — fused online-softmax attention; q is the caller's fp32
 // Q, k a TF32-rounded copy of K, vt the rounded V transposed to [b][dv][nk_pitch].

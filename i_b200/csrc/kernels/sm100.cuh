@@ -249,6 +249,15 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
+// ---- exchange between the threads of a warp that each hold a row ----
+
+// A warp's exchange buffer of 32 rows x 16 columns: four 16-byte units a row, placed so that eight
+// lanes that read or write either two whole rows or one unit of eight rows meet no bank twice.
+constexpr int kSwapFloats = 32 * 16;
+__device__ __forceinline__ float4* swap_at(float* swap, int row, int unit) {
+  return reinterpret_cast<float4*>(swap + row * 16 + ((unit ^ ((row >> 1) & 3)) << 2));
+}
+
 // ---- tcgen05.mma ----------------------------------------------------------
 
 enum class Kind { TF32, BF16 };

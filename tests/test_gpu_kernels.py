@@ -467,6 +467,26 @@ def run_contract(lib, torch, a, b, akm, bkm, precision, batch=None):
 
 
 @pytest.mark.parametrize("batch,m,n,k", [
+    (1, 33, 65, 1000),           # strips divided over clusters, a warp a row
+    (3, 40, 130, 77),            # a depth that is no multiple of eight, nothing on 16 bytes
+    (1, 300, 264, 1100),         # a CTA a row
+    (1, 5, 300, 8300)])          # rows too long to stay in registers, clusters of eight
+@pytest.mark.parametrize("akm,bkm", [(True, True), (True, False), (False, True), (False, False)])
+@pytest.mark.parametrize("precision,tol", [(F16, 1e-3), (BF16, 8e-3)])
+def test_contract_16_bit_operands_of_every_layout(lib, torch, batch, m, n, k, akm, bkm, precision, tol):
+    # Two operands rounded to 11 (8) bits: a product is off by at most 2^-10 (2^-7) of itself, the sum by less
+    # than that of the 2-norms of its row and column; rows of very different size keep their own scales.
+    a = rand((batch, m, k), 31) * (np.float32(10.0) ** np.linspace(-4, 4, m).astype(np.float32))[None, :, None]
+    b = rand((batch, n, k), 32) * (np.float32(10.0) ** np.linspace(3, -3, n).astype(np.float32))[None, :, None]
+    fa = a if akm else np.ascontiguousarray(a.transpose(0, 2, 1))
+    fb = b if bkm else np.ascontiguousarray(b.transpose(0, 2, 1))
+    got = run_contract(lib, torch, fa, fb, akm, bkm, precision, batch=batch)
+    want = a.astype(np.float64) @ b.astype(np.float64).transpose(0, 2, 1)
+    size = np.linalg.norm(a.astype(np.float64), axis=2)[:, :, None] * np.linalg.norm(b.astype(np.float64), axis=2)[:, None, :]
+    assert (np.abs(got - want) / size).max() <= tol
+
+
+@pytest.mark.parametrize("batch,m,n,k", [
     (1, 33, 31, 31), (1, 32, 32, 2048), (3, 70, 50, 515),        # the smallest tile, whole and cut along k
     (1, 8, 8000, 40), (8, 300, 300, 128),                        # the middle tiles
     (1, 1000, 1030, 257), (1, 1920, 2049, 129)])                 # the large ones
