@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -26,7 +27,7 @@ __device__ __forceinline__ float round_tf32(float x) {
 
 // out[c][r] = in[r][c] through a 64 x 64 tile in shared memory.  Whole tiles of 16-byte-aligned
 // arrays move as 16-byte accesses on both sides (a thread loads four neighbouring columns of a row
-// and stores four neighbouring rows of a column); ragged or unaligned tiles go element by element.
+// and stores four neighbouring rows of a column); unaligned arrays go element by element.
 template <bool ROUND>
 __global__ void __launch_bounds__(256)
 transpose_kernel(const float* __restrict__ in, float* __restrict__ out, size_t rows, size_t cols,
@@ -38,35 +39,54 @@ transpose_kernel(const float* __restrict__ in, float* __restrict__ out, size_t r
   out += batch * cols * out_pitch;
   const size_t c0 = static_cast<size_t>(blockIdx.x) * kT, r0 = static_cast<size_t>(blockIdx.y) * kT;
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const bool whole = vec && r0 + kT <= rows && c0 + kT <= cols;
-  if (whole) {
+  // Every load of a tile is in flight before the first is used, on ragged tiles too: one element after
+  // the other they took sixteen round trips, and the last row of tiles was most of the kernel (700 x
+  // 3000: 12.5 us, now 5.6).
+  if (vec) {
+    const size_t c = c0 + 4 * tx;                        // cols is a multiple of four
+    float4 v[4];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-      const int r = ty + 16 * p;
-      const float4 v = *reinterpret_cast<const float4*>(in + (r0 + r) * cols + c0 + 4 * tx);
-      tile[r][4 * tx + 0] = v.x;
-      tile[r][4 * tx + 1] = v.y;
-      tile[r][4 * tx + 2] = v.z;
-      tile[r][4 * tx + 3] = v.w;
+      const size_t r = r0 + ty + 16 * p;
+      v[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r < rows && c < cols) v[p] = *reinterpret_cast<const float4*>(in + r * cols + c);
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      float* at = &tile[ty + 16 * p][4 * tx];
+      at[0] = v[p].x; at[1] = v[p].y; at[2] = v[p].z; at[3] = v[p].w;
     }
   } else {
-    for (int e = threadIdx.x; e < kT * kT; e += 256) {
-      const int r = e / kT, c = e % kT;
-      if (r0 + r < rows && c0 + c < cols) tile[r][c] = in[(r0 + r) * cols + c0 + c];
+    float v[16];
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      const size_t r = r0 + threadIdx.x / kT + 4 * p, c = c0 + threadIdx.x % kT;
+      v[p] = r < rows && c < cols ? in[r * cols + c] : 0.0f;
     }
+#pragma unroll
+    for (int p = 0; p < 16; ++p) tile[threadIdx.x / kT + 4 * p][threadIdx.x % kT] = v[p];
   }
   __syncthreads();
-  if (whole) {
+  if (vec) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const int c = ty + 16 * p;
+      const size_t r = r0 + 4 * tx;
       float4 v = make_float4(tile[4 * tx + 0][c], tile[4 * tx + 1][c], tile[4 * tx + 2][c], tile[4 * tx + 3][c]);
       if (ROUND) v = make_float4(round_tf32(v.x), round_tf32(v.y), round_tf32(v.z), round_tf32(v.w));
-      *reinterpret_cast<float4*>(out + (c0 + c) * out_pitch + r0 + 4 * tx) = v;
+      float* at = out + (c0 + c) * out_pitch + r;
+      if (c0 + c < cols && r + 4 <= rows) {
+        *reinterpret_cast<float4*>(at) = v;
+      } else if (c0 + c < cols) {
+        if (r + 0 < rows) at[0] = v.x;
+        if (r + 1 < rows) at[1] = v.y;
+        if (r + 2 < rows) at[2] = v.z;
+      }
     }
   } else {
-    for (int e = threadIdx.x; e < kT * kT; e += 256) {
-      const int c = e / kT, r = e % kT;
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      const int c = threadIdx.x / kT + 4 * p, r = threadIdx.x % kT;
       if (r0 + r < rows && c0 + c < cols)
         out[(c0 + c) * out_pitch + r0 + r] = ROUND ? round_tf32(tile[r][c]) : tile[r][c];
     }
@@ -661,12 +681,13 @@ prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
 // over one power of two per row, which brings the row's largest magnitude into [2^14, 2^15) and goes to
 // `scale` for the epilogue to multiply back.  Bound by HBM: one read of fp32, one write of half that.
 //   stored [rows][k]: TPR threads a row, which stays in their registers up to 32 TPR values, so that the
-//     maximum and the conversion share one read;
+//     maximum and the conversion share one read (2048 x 2048 x 2048 in fp16: 21 us with a CTA a row and
+//     two loads in flight a thread, 10.5 with 64 threads and eight);
 //   stored [k][rows]: a strip of 32 rows (128 bytes of every line), its k range divided between the CTAs
 //     of a cluster where the strips alone are too few; the parts' maxima meet in distributed shared
 //     memory, the conversion reads the strip again (from L2) and turns it through shared memory.
 // Before, such an operand was transposed in fp32 first and the two converted one after the other:
-// 4096 x 4096 x 4096 with B stored k first, whole call in bf16 175 -> 139 us, in fp16 184 -> 171.
+// 4096 x 4096 x 4096 with B stored k first, whole call in bf16 175 -> 145 us, in fp16 184 -> 157.
 struct ContractOperand {
   const float* in;
   void* out;
@@ -795,8 +816,10 @@ prepare_contract_kernel(const ContractOperand a, const ContractOperand b, size_t
   const unsigned at = threadIdx.x % TPR;
   const bool vec = k % 4 == 0 && (reinterpret_cast<uintptr_t>(o.in) & 15u) == 0;
   const bool held = quads <= TPR * 8;
-  for (size_t r = static_cast<size_t>(block) * (256 / TPR) + threadIdx.x / TPR; r < rows;
-       r += static_cast<size_t>(o.blocks) * (256 / TPR)) {
+  constexpr unsigned kGroups = 256 / TPR;
+  for (size_t r0 = static_cast<size_t>(block) * kGroups; r0 < rows; r0 += static_cast<size_t>(o.blocks) * kGroups) {
+    const size_t r = r0 + threadIdx.x / TPR;
+    const bool live = r < rows;
     const float* src = o.in + r * k;
     uint16_t* dst = static_cast<uint16_t*>(o.out) + r * kp;
     float4 x[8];
@@ -805,9 +828,9 @@ prepare_contract_kernel(const ContractOperand a, const ContractOperand b, size_t
       for (int u = 0; u < 8; ++u) {
         const size_t c = (q0 + u * TPR) * 4;
         x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (vec && c < k) {
+        if (live && vec && c < k) {
           x[u] = __ldg(reinterpret_cast<const float4*>(src + c));
-        } else if (c < k) {
+        } else if (live && c < k) {
           x[u].x = src[c];
           if (c + 1 < k) x[u].y = src[c + 1];
           if (c + 2 < k) x[u].z = src[c + 2];
@@ -825,22 +848,23 @@ prepare_contract_kernel(const ContractOperand a, const ContractOperand b, size_t
           m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
       }
       m = warp_fold<IB_OP_MAX>(m);
-      if (TPR == 256) {
-        __syncthreads();                     // part_max may still be read for the row before
+      if (TPR > 32) {
+        __syncthreads();                     // part_max may still be read for the rows before
         if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = m;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < 8; ++w) m = fmaxf(m, part_max[w]);
+        for (int w = 0; w < TPR / 32; ++w) m = fmaxf(m, part_max[threadIdx.x / TPR * (TPR / 32) + w]);
       }
       const float scale = f16_scale_for(m);
       inv = 1.0f / scale;
-      if (at == 0) o.scale[r] = scale;
+      if (at == 0 && live) o.scale[r] = scale;
     }
     for (size_t q0 = at; q0 < quads; q0 += TPR * 8) {
       if (!SCALED || !held) fetch(q0);
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        if (q0 + u * TPR < quads) *reinterpret_cast<uint2*>(dst + (q0 + u * TPR) * 4) = pack4_16<SCALED>(x[u], inv);
+        if (live && q0 + u * TPR < quads)
+          *reinterpret_cast<uint2*>(dst + (q0 + u * TPR) * 4) = pack4_16<SCALED>(x[u], inv);
     }
   }
 }
@@ -965,8 +989,9 @@ int prepare_contract_operands(const float* a, bool a_kmajor, void* a16, float* a
                               size_t k, size_t kp, cudaStream_t s) {
   if (batch == 0 || m == 0 || n == 0 || k == 0) return 0;
   const bool scaled = a_scale != nullptr;
-  // A warp a row while it holds the row (1024 values); above that a CTA a row.
-  const int tpr = kp <= 1024 ? 32 : 256;
+  // As few threads a row as hold it (32 values each): the more loads a thread has in flight, the less the
+  // wait for the row's maximum shows.
+  const int tpr = kp <= 1024 ? 32 : kp <= 2048 ? 64 : kp <= 4096 ? 128 : 256;
   // A strip's k range is divided until there are about two CTAs an SM or a part has 128 lines left.
   auto strips = [&](size_t rows, bool kmajor) { return kmajor ? 0 : batch * ((rows + 31) / 32); };
   const size_t n_strips = strips(m, a_kmajor) + strips(n, b_kmajor);
@@ -992,8 +1017,14 @@ int prepare_contract_operands(const float* a, bool a_kmajor, void* a16, float* a
   cfg.stream = s;
   cfg.attrs = &cluster;
   cfg.numAttrs = parts > 1 ? 1 : 0;
-  auto* kernel = scaled ? (tpr == 32 ? &prepare_contract_kernel<true, 32> : &prepare_contract_kernel<true, 256>)
-                        : (tpr == 32 ? &prepare_contract_kernel<false, 32> : &prepare_contract_kernel<false, 256>);
+  auto pick = [tpr](auto is_scaled) {
+    constexpr bool kScaled = decltype(is_scaled)::value;
+    return tpr == 32   ? &prepare_contract_kernel<kScaled, 32>
+           : tpr == 64  ? &prepare_contract_kernel<kScaled, 64>
+           : tpr == 128 ? &prepare_contract_kernel<kScaled, 128>
+                        : &prepare_contract_kernel<kScaled, 256>;
+  };
+  auto* kernel = scaled ? pick(std::true_type{}) : pick(std::false_type{});
   if (cudaLaunchKernelEx(&cfg, kernel, oa, ob, batch, k, kp, parts) != cudaSuccess)
     return fail(std::string("prepare_contract_operands: ") + cudaGetErrorString(cudaGetLastError()));
   count_launch();

@@ -469,7 +469,8 @@ def run_contract(lib, torch, a, b, akm, bkm, precision, batch=None):
 @pytest.mark.parametrize("batch,m,n,k", [
     (1, 33, 65, 1000),           # strips divided over clusters, a warp a row
     (3, 40, 130, 77),            # a depth that is no multiple of eight, nothing on 16 bytes
-    (1, 300, 264, 1100),         # a CTA a row
+    (1, 300, 264, 1100), (2, 131, 70, 2300),     # two and four warps a row
+    (1, 33, 40, 4200),           # a CTA a row
     (1, 5, 300, 8300)])          # rows too long to stay in registers, clusters of eight
 @pytest.mark.parametrize("akm,bkm", [(True, True), (True, False), (False, True), (False, False)])
 @pytest.mark.parametrize("precision,tol", [(F16, 1e-3), (BF16, 8e-3)])

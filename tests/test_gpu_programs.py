@@ -378,6 +378,13 @@ def test_folds_of_leading_axes(ilang, oracle):
     assert np.array_equal(i(">abij~bj").exec_numpy(y), y.max(axis=(0, 2)))
 
 
+@pytest.mark.parametrize("shape", [(700, 3000), (64, 64), (65, 132), (63, 4), (1, 5), (700, 3002), (129, 1), (3, 70, 61), (3, 68, 100)])
+def test_transpose_of_ragged_tiles(ilang, shape):
+    x = np.arange(int(np.prod(shape)), dtype=np.float32).reshape(shape)
+    got = ilang.i("ij~ji" if len(shape) == 2 else "bij~bji").exec_numpy(x)
+    assert np.array_equal(got, np.swapaxes(x, -1, -2))
+
+
 def test_permutations_and_broadcasts_move_whole_lines(ilang):
     # Copies with the last two axes exchanged go through the tiled transpose; maps whose operands
     # are contiguous or constant along the innermost axis run four results at a time.  Results
