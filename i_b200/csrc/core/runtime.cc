@@ -800,10 +800,14 @@ int pipelined_host_attention(const i_program* program, const ShapeTable& shapes,
   const size_t block_rows = by_rows ? rows_per_block : dims.nq;
   const size_t prep_bytes =
       by_rows ? ib_attention_prepare_bytes(1, dims.nk, dims.d, dims.dv, precision) : 0;
+  // One workspace for every block.  The last block may hold fewer heads and need more of it: few heads
+  // of few queries have their keys divided between more CTAs, whose partial results it holds.
+  auto heads_bytes = [&](size_t heads) {
+    return ib_attention_workspace_bytes(heads, dims.nq, dims.nk, dims.d, dims.dv, dims.v_kmajor, precision);
+  };
   const size_t ws_bytes =
       by_rows ? ib_attention_run_workspace_bytes(1, block_rows, dims.nk, dims.dv)
-              : ib_attention_workspace_bytes(block_heads, dims.nq, dims.nk, dims.d, dims.dv,
-                                             dims.v_kmajor, precision);
+              : std::max(heads_bytes(block_heads), heads_bytes(dims.batch - (blocks - 1) * block_heads));
   float* prepared = by_rows ? dev.alloc(prep_bytes, &err) : nullptr;
   float* ws = dev.alloc(ws_bytes, &err);
   int rc = 0;

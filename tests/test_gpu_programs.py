@@ -247,6 +247,19 @@ def test_host_buffers_many_heads_pipelined_by_heads(ilang, oracle):
         assert max_rel_to_peak(got[h], oracle.attention_fused(q[h], k[h], v[h])) <= 5e-3
 
 
+@pytest.mark.parametrize("heads,nq,nk", [
+    (55, 8, 12288), (41, 3, 16384), (86, 8, 8192),      # blocks of 7, 6, 11 heads, then a block of 6, 5, 9 that needs more
+    (9, 2, 40000), (17, 1, 9000)])                      # a last block of one head
+def test_host_buffers_few_queries_of_uneven_head_counts(ilang, heads, nq, nk):
+    # Blocks of heads share one workspace, and a smaller last block may be the one that needs most of it.
+    q, k, v = rand((heads, nq, 4), 81), rand((heads, nk, 4), 82), rand((heads, nk, 4), 83)
+    f = batched_readme_attention(ilang).set_precision("tf32")
+    got = f.exec_numpy(q, k, v)
+    assert max_rel_to_peak(got, np_attention(q, k, v)) <= 1e-5        # fp32: up to eight queries
+    out = np.empty_like(got)
+    assert np.array_equal(f.into(out, q, k, v), got)
+
+
 def test_softmax_component_config2_slice(ilang, oracle):
     i, I = ilang.i, ilang.I
     sm = ((I & i(">ij~i | i:16,j:16 | jii'j'")) >> i("ij-i~ij | i:16,j:16 | 1jii'j'")) \
