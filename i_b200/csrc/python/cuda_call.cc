@@ -3,13 +3,17 @@
 // What bounds a small call is the host: describing four tensors through ctypes (a shape array, a
 // struct and a few attribute look-ups each) took 14-18 us of Python where the launch itself takes
 // two.  Here the tensors are read through torch's own C++ type, so a call costs about 1 us besides
-// the runtime's.  The functions handle the common case only: every argument a contiguous float32
-// CUDA tensor on one device.  For anything else they return None before doing anything, and the
-// caller takes the general route, which also words the errors.
+// the runtime's.  The functions handle the common case only: every argument a dense, contiguous float32
+// CUDA tensor with memory of its own, on one device.  For anything else (sparse layouts, fake tensors and
+// other subclasses that dispatch in Python, functorch's wrappers under vmap or grad) they return None
+// before doing anything, and the caller takes the general route, which also words the errors.  What torch
+// throws on the way becomes the Python exception it stands for: nothing may leave a C function.
 //
 // The library is reached through function addresses handed over once (bind), so it stays the one
 // ilang.py loaded.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -37,9 +41,10 @@ struct Described {
 
   // False when `t` is not what this file handles; `device` is the first tensor's, or -1.
   bool add(const at::Tensor& t, int* device) {
-    if (count == kMostTensors || !t.is_cuda() || t.scalar_type() != at::kFloat || t.dim() > kMostRank ||
-        !t.is_contiguous())
-      return false;
+    if (count == kMostTensors || !t.defined() || !t.is_cuda() || t.scalar_type() != at::kFloat) return false;
+    // Before anything that needs a storage: wrappers have none, fake tensors dispatch in Python.
+    if (t.layout() != at::kStrided || !t.has_storage() || t.key_set().has(c10::DispatchKey::Python)) return false;
+    if (t.dim() > kMostRank || !t.is_contiguous()) return false;
     if (*device < 0) *device = t.get_device();
     if (t.get_device() != *device) return false;
     const auto sizes = t.sizes();
@@ -97,72 +102,69 @@ const i_program* program_of(PyObject* o) { return static_cast<const i_program*>(
 // Returns what Component.into returns, or None when the call is not of this file's kind.
 PyObject* into(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 3 || !PyTuple_Check(args[2])) Py_RETURN_NONE;
-  PyObject* given = args[1];
-  int device = -1;
-  Described in, out;
-  if (!describe_all(args[2], &in, &device)) Py_RETURN_NONE;
-  PyObject* many = nullptr;            // owned: the outputs as a tuple
-  if (PyTuple_Check(given) || PyList_Check(given)) {
-    many = PySequence_Tuple(given);
-    if (!many) return nullptr;
+  try {
+    PyObject* given = args[1];
+    int device = -1;
+    Described in, out;
+    if (!describe_all(args[2], &in, &device)) Py_RETURN_NONE;
+    THPObjectPtr many;                   // the outputs as a tuple
+    if (PyTuple_Check(given) || PyList_Check(given)) {
+      many = PySequence_Tuple(given);
+      if (!many) return nullptr;
+    }
+    const bool described = many ? describe_all(many, &out, &device) : out.add(given, &device);
+    if (!described || device < 0) Py_RETURN_NONE;
+    if (launch(program_of(args[0]), in, out, device)) return fail();
+    if (!many) return Py_NewRef(given);
+    return PyTuple_GET_SIZE(many.get()) == 1 ? Py_NewRef(PyTuple_GET_ITEM(many.get(), 0)) : many.release();
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
   }
-  const bool described = many ? describe_all(many, &out, &device) : out.add(given, &device);
-  if (!described || device < 0) {
-    Py_XDECREF(many);
-    Py_RETURN_NONE;
-  }
-  if (launch(program_of(args[0]), in, out, device)) {
-    Py_XDECREF(many);
-    return fail();
-  }
-  if (!many) return Py_NewRef(given);
-  if (PyTuple_GET_SIZE(many) != 1) return many;
-  PyObject* only = Py_NewRef(PyTuple_GET_ITEM(many, 0));
-  Py_DECREF(many);
-  return only;
 }
 
 // exec(program, inputs): allocates the outputs and runs; what exec_torch returns, or None when the
 // call is not of this file's kind.
 PyObject* exec(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 2 || !PyTuple_Check(args[1])) Py_RETURN_NONE;
-  int device = -1;
-  Described in, out;
-  if (!describe_all(args[1], &in, &device) || device < 0) Py_RETURN_NONE;
-  const i_program* program = program_of(args[0]);
-  const size_t count = g_lib.output_count(program);
-  if (count == 0 || count > kMostTensors) Py_RETURN_NONE;
-  size_t ranks[kMostTensors], shapes[kMostTensors][kMostRank];
-  size_t* rows[kMostTensors];
-  if (g_lib.output_ranks(program, ranks)) return fail();
-  for (size_t o = 0; o < count; ++o) {
-    if (ranks[o] > kMostRank) Py_RETURN_NONE;
-    rows[o] = shapes[o];
-  }
-  if (g_lib.output_shapes(program, in.tensors, static_cast<size_t>(in.count), rows)) return fail();
-  PyObject* made = count == 1 ? nullptr : PyTuple_New(static_cast<Py_ssize_t>(count));
-  if (count != 1 && !made) return nullptr;
-  at::Tensor first;
   try {
+    int device = -1;
+    Described in, out;
+    if (!describe_all(args[1], &in, &device) || device < 0) Py_RETURN_NONE;
+    const i_program* program = program_of(args[0]);
+    const size_t count = g_lib.output_count(program);
+    if (count == 0 || count > kMostTensors) Py_RETURN_NONE;
+    size_t ranks[kMostTensors], shapes[kMostTensors][kMostRank];
+    size_t* rows[kMostTensors];
+    if (g_lib.output_ranks(program, ranks)) return fail();
+    for (size_t o = 0; o < count; ++o) {
+      if (ranks[o] > kMostRank) Py_RETURN_NONE;
+      rows[o] = shapes[o];
+    }
+    if (g_lib.output_shapes(program, in.tensors, static_cast<size_t>(in.count), rows)) return fail();
+    THPObjectPtr made;                   // several outputs as a tuple
+    if (count != 1 && !(made = PyTuple_New(static_cast<Py_ssize_t>(count)))) return nullptr;
+    at::Tensor first;
     const auto options = at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, static_cast<c10::DeviceIndex>(device));
     for (size_t o = 0; o < count; ++o) {
       int64_t dims[kMostRank];
       for (size_t d = 0; d < ranks[o]; ++d) dims[d] = static_cast<int64_t>(shapes[o][d]);
       at::Tensor t = at::empty(at::IntArrayRef(dims, ranks[o]), options);
-      out.add(t, &device);
-      if (made) PyTuple_SET_ITEM(made, static_cast<Py_ssize_t>(o), THPVariable_Wrap(t));
-      else first = std::move(t);
+      if (!out.add(t, &device)) Py_RETURN_NONE;      // a dispatch mode made something else of it
+      if (made) {
+        PyObject* wrapped = THPVariable_Wrap(t);
+        if (!wrapped) return nullptr;
+        PyTuple_SET_ITEM(made.get(), static_cast<Py_ssize_t>(o), wrapped);
+      } else {
+        first = std::move(t);
+      }
     }
-  } catch (const std::exception& e) {
-    Py_XDECREF(made);
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+    if (launch(program, in, out, device)) return fail();
+    return made ? made.release() : THPVariable_Wrap(first);
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
     return nullptr;
   }
-  if (launch(program, in, out, device)) {
-    Py_XDECREF(made);
-    return fail();
-  }
-  return made ? made : THPVariable_Wrap(first);
 }
 
 PyMethodDef kMethods[] = {
