@@ -40,7 +40,8 @@ struct Described {
   int count = 0;
 
   // False when `t` is not what this file handles; `device` is the first tensor's, or -1.
-  bool add(const at::Tensor& t, int* device) {
+  // The address of an output is asked for as one to write to: a lazy clone then gets memory of its own.
+  bool add(const at::Tensor& t, int* device, bool output) {
     if (count == kMostTensors || !t.defined() || !t.is_cuda() || t.scalar_type() != at::kFloat) return false;
     // Before anything that needs a storage: wrappers have none, fake tensors dispatch in Python.
     if (t.layout() != at::kStrided || !t.has_storage() || t.key_set().has(c10::DispatchKey::Python)) return false;
@@ -49,17 +50,20 @@ struct Described {
     if (t.get_device() != *device) return false;
     const auto sizes = t.sizes();
     for (size_t d = 0; d < sizes.size(); ++d) extents[count][d] = static_cast<size_t>(sizes[d]);
-    tensors[count] = i_tensor{static_cast<const float*>(t.const_data_ptr()), extents[count], sizes.size()};
+    tensors[count] = i_tensor{static_cast<const float*>(output ? t.mutable_data_ptr() : t.const_data_ptr()), extents[count],
+                              sizes.size()};
     ++count;
     return true;
   }
-  bool add(PyObject* o, int* device) { return THPVariable_Check(o) && add(THPVariable_Unpack(o), device); }
+  bool add(PyObject* o, int* device, bool output) {
+    return THPVariable_Check(o) && add(THPVariable_Unpack(o), device, output);
+  }
 };
 
-bool describe_all(PyObject* tuple, Described* out, int* device) {
+bool describe_all(PyObject* tuple, Described* out, int* device, bool outputs) {
   const Py_ssize_t n = PyTuple_GET_SIZE(tuple);
   for (Py_ssize_t i = 0; i < n; ++i)
-    if (!out->add(PyTuple_GET_ITEM(tuple, i), device)) return false;
+    if (!out->add(PyTuple_GET_ITEM(tuple, i), device, outputs)) return false;
   return true;
 }
 
@@ -106,13 +110,13 @@ PyObject* into(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyObject* given = args[1];
     int device = -1;
     Described in, out;
-    if (!describe_all(args[2], &in, &device)) Py_RETURN_NONE;
+    if (!describe_all(args[2], &in, &device, false)) Py_RETURN_NONE;
     THPObjectPtr many;                   // the outputs as a tuple
     if (PyTuple_Check(given) || PyList_Check(given)) {
       many = PySequence_Tuple(given);
       if (!many) return nullptr;
     }
-    const bool described = many ? describe_all(many, &out, &device) : out.add(given, &device);
+    const bool described = many ? describe_all(many, &out, &device, true) : out.add(given, &device, true);
     if (!described || device < 0) Py_RETURN_NONE;
     if (launch(program_of(args[0]), in, out, device)) return fail();
     if (!many) return Py_NewRef(given);
@@ -130,7 +134,7 @@ PyObject* exec(PyObject*, PyObject* const* args, Py_ssize_t n) {
   try {
     int device = -1;
     Described in, out;
-    if (!describe_all(args[1], &in, &device) || device < 0) Py_RETURN_NONE;
+    if (!describe_all(args[1], &in, &device, false) || device < 0) Py_RETURN_NONE;
     const i_program* program = program_of(args[0]);
     const size_t count = g_lib.output_count(program);
     if (count == 0 || count > kMostTensors) Py_RETURN_NONE;
@@ -150,7 +154,7 @@ PyObject* exec(PyObject*, PyObject* const* args, Py_ssize_t n) {
       int64_t dims[kMostRank];
       for (size_t d = 0; d < ranks[o]; ++d) dims[d] = static_cast<int64_t>(shapes[o][d]);
       at::Tensor t = at::empty(at::IntArrayRef(dims, ranks[o]), options);
-      if (!out.add(t, &device)) Py_RETURN_NONE;      // a dispatch mode made something else of it
+      if (!out.add(t, &device, true)) Py_RETURN_NONE;      // a dispatch mode made something else of it
       if (made) {
         PyObject* wrapped = THPVariable_Wrap(t);
         if (!wrapped) return nullptr;

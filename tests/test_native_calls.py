@@ -105,3 +105,14 @@ def test_what_the_native_route_refuses(ilang, torch):
         assert np.array_equal(f.exec_numpy(given), 0.0 - want)
     with pytest.raises(TypeError, match="float32"):
         f.into(np.empty((6, 10), np.float64), want)
+
+
+@pytest.mark.gpu
+def test_an_output_that_shares_memory_until_written(ilang, torch):
+    # A lazy clone shares its source's memory; writing it as an output must not write the source.
+    f = ilang.i("-ij~ij")
+    x, source = torch.randn(6, 10, device="cuda"), torch.zeros(6, 10, device="cuda")
+    for outputs in (torch._lazy_clone(source), [torch._lazy_clone(source)]):
+        assert torch.equal(f.into(outputs, x), 0.0 - x) and not source.any()
+    lazy = torch._lazy_clone(x)
+    assert torch.equal(f.exec_torch(lazy), 0.0 - x)
