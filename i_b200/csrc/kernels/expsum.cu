@@ -10,6 +10,7 @@
 // shared memory.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -218,7 +219,6 @@ extern "C" int ib_row_expsum(const float* x, float* y, size_t rows, size_t cols,
   if (!y || (!x && cols != 0)) return fail("ib_row_expsum: null pointer");
   if (n_post < 0 || n_post > IB_MAX_CHAIN_OPS || (n_post > 0 && !post_ops))
     return fail("ib_row_expsum: between 0 and " + std::to_string(IB_MAX_CHAIN_OPS) + " operators");
-  if (rows > 0x7fffffffu / 8) return fail("ib_row_expsum: too many rows");
   GemmEpilogue post;
   post.n_ops = n_post;
   for (int k = 0; k < n_post; ++k) {
@@ -231,11 +231,18 @@ extern "C" int ib_row_expsum(const float* x, float* y, size_t rows, size_t cols,
   // A warp per row up to 2048 columns (as the plain row folds): a CTA's 256 threads would hold fewer
   // than two 16-byte loads each.
   if (cols <= 2048) {
-    const unsigned blocks = static_cast<unsigned>((rows + kWarps - 1) / kWarps);
-    if (vec) row_expsum_warp<true><<<blocks, kThreads, 0, s>>>(x, y, rows, cols, post);
-    else row_expsum_warp<false><<<blocks, kThreads, 0, s>>>(x, y, rows, cols, post);
-    return check_launch("ib_row_expsum");
+    // As many rows a launch as its grid holds (2^34; a loop over rows inside the kernel cost short rows 10 %).
+    constexpr size_t kMost = static_cast<size_t>(0x7fffffff) * kWarps;
+    for (size_t r0 = 0; r0 < rows; r0 += kMost) {
+      const size_t n = std::min(rows - r0, kMost);
+      const unsigned blocks = static_cast<unsigned>((n + kWarps - 1) / kWarps);
+      if (vec) row_expsum_warp<true><<<blocks, kThreads, 0, s>>>(x + r0 * cols, y + r0, n, cols, post);
+      else row_expsum_warp<false><<<blocks, kThreads, 0, s>>>(x + r0 * cols, y + r0, n, cols, post);
+      if (int rc = check_launch("ib_row_expsum")) return rc;
+    }
+    return 0;
   }
+  if (rows > 0x7fffffff) return fail("ib_row_expsum: more than 2^31 - 1 rows of more than 2048 columns");
   // Rows too few to give every SM several CTAs are cut into up to eight parts of at least 4096 columns.
   size_t parts = static_cast<size_t>(kNumSMs) * 4 / rows;
   if (parts > cols / 4096) parts = cols / 4096;

@@ -568,6 +568,17 @@ def test_row_sum_of_shifted_exponentials(ilang, rows, cols):
     assert max_rel_elementwise(got, want) <= 1e-5 and np.array_equal(zero, np.zeros(rows, np.float32))
 
 
+def test_row_sum_of_shifted_exponentials_of_very_many_rows(ilang):
+    # 2^28 + 3 rows, more than an eighth of the CTAs that a grid holds: 2 GiB of x and 1 GiB of sums.
+    import torch
+    i, I = ilang.i, ilang.I
+    denom = (I & i(">ij~i")) >> (i("ij-i~ij") >> i("^ij~ij") >> i("+ij~i"))
+    x = torch.rand(2 ** 28 + 3, 2, device="cuda")
+    got = denom.into(torch.full((x.shape[0],), float("nan"), device="cuda"), x)
+    got -= 1 + torch.exp(-(x[:, 0] - x[:, 1]).abs())
+    assert got.abs().max().item() <= 1e-5
+
+
 def test_row_sum_of_shifted_exponentials_special_values(ilang):
     # As in the reference's chain: a row of -inf alone and a row with +inf or NaN give NaN.
     i, I = ilang.i, ilang.I
