@@ -1,5 +1,6 @@
 // ib_contract and ib_attention: precision choice, workspace carving and the
 // layout fix-ups that give the tensor-core kernels K-major operands.
+#include <algorithm>
 #include <initializer_list>
 #include "common.cuh"
 #include "kernels.h"
@@ -234,7 +235,11 @@ extern "C" size_t ib_contract_workspace_bytes(size_t batch, size_t m, size_t n, 
     return copies > 1 ? carve_bytes(batch * copies * m * n) : 0;
   }();
   if (!wants_tensor(precision, flop)) return fp32_bytes;
-  if (precision == IB_PRECISION_AUTO && contract_prefers_f16(m, n, k)) precision = IB_PRECISION_F16;
+  // AUTO takes the fp16 arm only with a 256-byte aligned workspace, else the TF32 arm, whose fp32
+  // transposes may need more.
+  if (precision == IB_PRECISION_AUTO && contract_prefers_f16(m, n, k))
+    return std::max(ib_contract_workspace_bytes(batch, m, n, k, a_kmajor, b_kmajor, IB_PRECISION_F16),
+                    ib_contract_workspace_bytes(batch, m, n, k, a_kmajor, b_kmajor, IB_PRECISION_TF32));
   if (precision == IB_PRECISION_F16) {
     // fp16 copies of both operands plus one scale per row.
     const size_t kp = round_up(k, 8);

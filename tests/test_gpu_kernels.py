@@ -604,6 +604,18 @@ def test_contract_auto_large_deep_shape(lib, torch):
         assert err <= TOL_TF32, (with_ws, err)
 
 
+def test_contract_auto_with_an_unaligned_workspace(lib, torch):
+    # Off 256 bytes AUTO takes the TF32 arm, whose transposes have to fit the workspace it asked for.
+    m, n, k = 4096, 4224, 2048
+    a, b = torch.randn(k, m, device="cuda"), torch.randn(k, n, device="cuda")
+    c = torch.full((m, n), float("nan"), device="cuda")
+    wb = lib.ib_contract_workspace_bytes(1, m, n, k, 0, 0, 0)
+    ws = torch.empty(wb + 256, dtype=torch.uint8, device="cuda")
+    ok(lib, lib.ib_contract(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, m, n, k, 0, 0, 0, ws.data_ptr() + 16, wb, None))
+    ref = a.double().t() @ b.double()
+    assert ((c.double() - ref).abs().max() / ref.abs().max()).item() <= TOL_TF32
+
+
 def test_contract_tf32_batched(lib, oracle, torch):
     a, b = rand((3, 150, 64), 13), rand((3, 90, 64), 14)
     got = run_contract(lib, torch, a, b, True, True, TF32, batch=3)

@@ -113,3 +113,13 @@ def test_workspace_sizes_of_folds_and_split_contractions(lib):
     assert lib.ib_contract_workspace_bytes(1, 2048, 2048, 4096, 1, 1, FP32) == 0
     assert lib.ib_contract_workspace_bytes(1, 8192, 1, 8192, 1, 1, AUTO) == 0
     assert lib.ib_contract_workspace_bytes(1, 8192, 1, 8192, 0, 1, AUTO) > 0      # [k][rows]: slabs' partial sums
+
+
+@pytest.mark.parametrize("akm", [0, 1])
+@pytest.mark.parametrize("bkm", [0, 1])
+def test_workspace_of_auto_serves_either_tensor_arm(lib, akm, bkm):
+    # Where AUTO prefers the fp16 arm it takes the TF32 arm if the workspace is not aligned for the former.
+    declare(lib)
+    for m, n, k in ((4096, 4096, 2048), (4096, 4096, 4096), (5000, 4100, 3001), (8192, 8192, 4096)):
+        size = {p: lib.ib_contract_workspace_bytes(1, m, n, k, akm, bkm, p) for p in (AUTO, TF32, 5)}
+        assert size[AUTO] >= max(size[TF32], size[5])
