@@ -1797,21 +1797,41 @@ long long granule_tiles(size_t kv_granule, long long kv_tiles) {
   return t < 1 ? 1 : (t > kv_tiles ? kv_tiles : t);
 }
 
-// Whether the key ranges of the row tiles that do not fill a wave are divided between the CTAs.  In
-// units of one key tile's time on an SM (1.0 - 1.2 us at d = 128): a piece of a row tile costs its key
-// tiles plus about 4 (Q staged, pipeline filled, O read out); divided, the last wave's key tiles
-// spread over all CTAs, which then handle two pieces each, write partial results and leave a merge
-// kernel to run, together about 24.  Measured on B200 (fp16 arm, back to back, divided / whole): one head of
-// 16384 170 / 164 us, of 12800 115 / 119, of 8192 66 / 81; 64 heads x 2048 276 / 262; 9 x 2048 58 / 42;
-// 40 x 700 66 / 55; 2048 queries x 16384 keys 66 / 140.
-bool divides_keys(long long units, long long kv_tiles, long long sms) {
-  constexpr double kPiece = 4.0, kDivided = 24.0;
-  const long long waves = units / sms, tail = units % sms;
-  if (tail == 0) return false;
-  const double whole = static_cast<double>(waves + 1) * (kv_tiles + kPiece);
-  const double divided = static_cast<double>(waves) * (kv_tiles + kPiece) +
-                         static_cast<double>(tail) * kv_tiles / sms + kDivided;
-  return divided < whole;
+// Whether the key ranges of the row tiles that do not fill a wave are divided between the CTAs: whole, the
+// last wave takes as long as one row tile; divided, its key tiles spread over all CTAs, which write partial
+// results and leave a merge kernel to run.  The first costs key tiles and the second a fixed time, so the line
+// lies elsewhere for each arm: a key tile takes 1.05 us on 16-bit operands, 1.6 with TF32 logits, 1.9 in
+// TF32 throughout, whatever the width of a head.  The fixed time grows with the width of the values and the
+// number of CTAs, and is less where every CTA has a single piece (its share divides a row tile's keys).
+// Measured on B200, whole / divided in us:
+//   heads x queries x keys x width   fp16           bf16           TF32 x fp16    TF32
+//   1 x 16384 x 16384 x 128          145 / 153      155 / 159      235 / 224      265 / 248
+//   1 x 12800 x 12800 x 128          115 / 106      112 / 101      171 / 139      196 / 156
+//   1 x 2048 x 2048 x 128            30.1 / 33.1    26.9 / 31.0    39.2 / 35.1    41.2 / 32.9
+//   1 x 2048 x 2048 x 32             29.0 / 24.8    26.9 / 20.7    35.1 / 23.0    37.2 / 20.8
+//   1 x 512 x 1024 x 64              20.6 / 19.0    17.3 / 15.4    22.9 / 18.1    22.9 / 16.6
+//   6 x 1500 x 2300 x 64             33.0 / 37.0    30.6 / 33.0    41.7 / 37.5    45.3 / 37.2
+//   9 x 2048 x 2048 x 128            39.2 / 56.2    35.1 / 50.8    49.1 / 62.6    51.5 / 63.1
+//   64 x 2048 x 2048 x 128           219 / 238      193 / 218      331 / 346      326 / 341
+// Over 460 such pairs (1 to 1024 row tiles, 4 to 512 key tiles, widths 32 to 128, the four arms) the rule
+// takes the slower form in 11, where the two lie 2 to 10 % apart (once 20 %: one row tile of nine key tiles).
+// `coarse`: key tiles per granule at which a range may be cut.
+bool divides_keys(long long units, long long kv_tiles, long long coarse, long long sms, AttentionArm arm, size_t dv) {
+  const long long granules = (kv_tiles + coarse - 1) / coarse;
+  if (units % sms == 0 || granules < 2) return false;
+  const bool narrow = arm == AttentionArm::F16 || arm == AttentionArm::BF16;
+  const double tile_us = narrow ? 1.05 : arm == AttentionArm::MIXED ? 1.60 : 1.90;
+  const double crowded = narrow ? 1.07 : 1.0;               // all SMs against the few of a last wave
+  const long long ctas = choose_ctas(units, kv_tiles, granules, static_cast<int>(sms));
+  const long long waves = units / ctas, left = (units - waves * ctas) * granules, share = left / ctas;
+  const bool one_piece = left % ctas == 0 && share > 0 && granules % share == 0;
+  const double width = static_cast<double>(dv), crowd = static_cast<double>(ctas) / kNumSMs;
+  const double fixed_us = (one_piece ? 2.0 + 0.12 * width * crowd : 5.5 + 0.06 * width + (2.0 + 0.025 * width) * crowd) *
+                          (narrow ? 1.0 : 0.88);
+  const double last = static_cast<double>((share + (left % ctas ? 1 : 0)) * coarse);
+  const double longest = static_cast<double>(waves * kv_tiles) + crowded * last;
+  const double whole = static_cast<double>((units + sms - 1) / sms * kv_tiles);
+  return longest * tile_us + fixed_us < whole * tile_us;
 }
 
 // SMs the persistent kernel leaves free (for a communication kernel running next to it).
@@ -1909,9 +1929,8 @@ int attention_tcgen05(const float* q, const void* k, const void* vt, float* o, s
   const long long units = static_cast<long long>(p.q_tiles) * p.batch;
   // Where a row tile's key range may be cut between CTAs: at multiples of the caller's granule
   // (whole 128-key tiles); a granule of the whole range or more means never.
-  p.coarse = static_cast<int>(divides_keys(units, p.kv_tiles, device_sms())
-                                  ? granule_tiles(kv_granule, p.kv_tiles)
-                                  : static_cast<long long>(p.kv_tiles));
+  const long long coarse = granule_tiles(kv_granule, p.kv_tiles);
+  p.coarse = static_cast<int>(divides_keys(units, p.kv_tiles, coarse, device_sms(), arm, dv) ? coarse : p.kv_tiles);
   p.kv_coarse = (p.kv_tiles + p.coarse - 1) / p.coarse;
   const int ctas = choose_ctas(units, p.kv_tiles, p.kv_coarse, device_sms());
   p.ctas = ctas;

@@ -1018,3 +1018,32 @@ def test_attention_direct_fp32(lib, torch, batch, nq, nk, d, dv, scale):
     p = np.exp(s - s.max(axis=2, keepdims=True))
     want = np.einsum("bqk,bkv->bqv", p / p.sum(axis=2, keepdims=True), v.astype(np.float64))
     assert max_rel_to_peak(out.cpu().numpy(), want) <= TOL_FP32
+
+
+@pytest.mark.parametrize("precision,tol", [(F16, TOL_TF32), (BF16, TOL_BF16), (TF32_F16, TOL_TF32), (TF32, TOL_TF32)])
+@pytest.mark.parametrize("batch,nq,nk,d,divided", [
+    (1, 2048, 2048, 128, (TF32_F16, TF32)),             # sixteen row tiles of sixteen key tiles
+    (1, 2000, 2040, 32, (F16, BF16, TF32_F16, TF32)),   # narrow heads: partial results cost less
+    (6, 1500, 2300, 64, (TF32_F16, TF32)),
+    (1, 6100, 6100, 128, (F16, BF16, TF32_F16, TF32)),
+    (9, 2048, 2048, 128, ()),                           # four SMs without a row tile
+    (20, 1024, 1000, 128, ())])                         # two waves, the second nearly empty
+def test_attention_divides_keys_where_the_arm_gains(lib, torch, precision, tol, batch, nq, nk, d, divided):
+    # Divided, the call has a merge kernel; a granule of all keys forbids it.  Results agree either way.
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nq + nk + d)
+    q = torch.randn(batch, nq, d, device="cuda", generator=g) * d ** -0.5
+    k, v = (torch.randn(batch, nk, d, device="cuda", generator=g) for _ in range(2))
+    want = torch.softmax(q.double() @ k.double().transpose(1, 2), -1) @ v.double()
+    ws_bytes = lib.ib_attention_workspace_bytes(batch, nq, nk, d, d, 0, precision)
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device="cuda")
+    launches = []
+    for granule in (0, nk):
+        o = torch.full((batch, nq, d), float("nan"), device="cuda")
+        before = lib.i_b200_launch_count()
+        ok(lib, lib.ib_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), batch, nq, nk, d, d, 0,
+                                 precision, granule, ws.data_ptr(), ws_bytes, None))
+        launches.append(lib.i_b200_launch_count() - before)
+        torch.cuda.synchronize()
+        assert ((o.double() - want).abs().max() / want.abs().max()).item() <= tol
+    assert launches[0] - launches[1] == (precision in divided)
