@@ -731,12 +731,13 @@ attention_tf32_kernel(const __grid_constant__ CUtensorMap map_k,
       }
       // S -> exponent units: log2(e), times the scales Q's row and K's tile were stored over.
       // K's scales come from the preparation kernel; every read of them follows an S that was
-      // computed from its K, so the kernel has completed.
+      // computed from its K, so the kernel has completed.  Plain loads, never the read-only path: that
+      // kernel may still have been running when this one started.
       float mul = kLog2E32;
       if (G::kScaledQk) {
         const float* ks = p.k_tile_scale + static_cast<size_t>(b) * p.kv_tiles + kv_lo + jj;
-        const float here = jj == 0 ? __ldg(ks) : ks_ahead;
-        if (jj + 1 < n_kv) ks_ahead = __ldg(ks + 1);
+        const float here = jj == 0 ? *ks : ks_ahead;
+        if (jj + 1 < n_kv) ks_ahead = ks[1];
         mul = row_mul * here;
       }
       float mx = -CUDART_INF_F;
@@ -1380,7 +1381,7 @@ attention_pipelined_kernel(const __grid_constant__ CUtensorMap map_k,
           const int col0 = (pc.kv_lo + jj) * kBKV;
           float mx = -CUDART_INF_F;
           float mul = row_mul;
-          if (G::kScaledQk) mul *= __ldg(p.k_tile_scale + static_cast<size_t>(b) * p.kv_tiles + pc.kv_lo + jj);
+          if (G::kScaledQk) mul *= p.k_tile_scale[static_cast<size_t>(b) * p.kv_tiles + pc.kv_lo + jj];
           // One block of 32 columns at a time (this warpgroup runs on 64 registers).
 #pragma unroll 1
           for (int c = 0; c < kBKV; c += 32) {
@@ -1524,9 +1525,9 @@ attention_pipelined_kernel(const __grid_constant__ CUtensorMap map_k,
         float mul = kLog2E32;
         if (G::kScaledQk) {
           const float* ks = p.k_tile_scale + static_cast<size_t>(b) * p.kv_tiles + kv_lo + jj;
-          const float here = have_scale ? ks_ahead : __ldg(ks);
+          const float here = have_scale ? ks_ahead : *ks;
           have_scale = jj + 2 < n_kv;
-          if (have_scale) ks_ahead = __ldg(ks + 2);
+          if (have_scale) ks_ahead = ks[2];
           mul = row_mul * here;
         }
         const float m_used = sh->pub_m[t & 3][r];

@@ -79,17 +79,22 @@ struct EpilogueRows {
   int rows;              // rows of the result from there on
   int n;
   bool vec;              // n and c allow 16-byte accesses
-  const float* rs;       // row scales from the first row on, or null
-  const float* cs;       // column scales of the batch entry, or null
+  // Row scales from the first row on and column scales of the batch entry, or null.  The conversion may
+  // still be storing them when this kernel starts, so they are read by plain loads behind the wait for it,
+  // never through the read-only path.
+  const float* rs;
+  const float* cs;
 };
 
+template <bool READ_ONLY = true>
 __device__ __forceinline__ void load_columns(float (&t)[4], const float* p, int col, int n, bool vec) {
   if (vec && col < n && (reinterpret_cast<uintptr_t>(p + col) & 15u) == 0) {
-    const float4 x = __ldg(reinterpret_cast<const float4*>(p + col));
+    const float4* at = reinterpret_cast<const float4*>(p + col);
+    const float4 x = READ_ONLY ? __ldg(at) : *at;
     t[0] = x.x; t[1] = x.y; t[2] = x.z; t[3] = x.w;
   } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) t[j] = col + j < n ? __ldg(p + col + j) : 0.0f;
+    for (int j = 0; j < 4; ++j) t[j] = col + j >= n ? 0.0f : READ_ONLY ? __ldg(p + col + j) : p[col + j];
   }
 }
 
@@ -112,7 +117,7 @@ __device__ __forceinline__ void look_ahead(ColumnsAhead& x, const GemmEpilogue& 
   const int col = col0 + (threadIdx.x & 3) * 4;
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
-    if (at.cs) load_columns(x.scale[part], at.cs, col + part * 16, at.n, at.vec);
+    if (at.cs) load_columns<false>(x.scale[part], at.cs, col + part * 16, at.n, at.vec);
     if (per_column >= 0) load_columns(x.operand[part], e.operand[e.which[per_column]], col + part * 16, at.n, at.vec);
   }
 }
@@ -228,7 +233,7 @@ template <int BN, Kind KIND>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  float* __restrict__ c, int m, int n, int k, int batch, int* status,
-                 const float* __restrict__ row_scale, const float* __restrict__ col_scale,
+                 const float* row_scale, const float* col_scale,
                  int f16_operands, int group_n, const __grid_constant__ GemmEpilogue epilogue) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -353,7 +358,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       float rs[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        rs[i] = row_scale && (lane >> 2) + i * 8 < at.rows ? __ldg(at.rs + (lane >> 2) + i * 8) : 1.0f;
+        rs[i] = row_scale && (lane >> 2) + i * 8 < at.rows ? at.rs[(lane >> 2) + i * 8] : 1.0f;
       ok = mbar_wait(&acc_full[acc], acc_phase, abort, status, 104);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -423,7 +428,7 @@ template <Kind KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  float* __restrict__ c, int m, int n, int k, int batch, int* status,
-                 const float* __restrict__ row_scale, const float* __restrict__ col_scale,
+                 const float* row_scale, const float* col_scale,
                  int f16_operands, int group_n, const __grid_constant__ GemmEpilogue epilogue) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -594,7 +599,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       float rs[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        rs[i] = row_scale && (lane >> 2) + i * 8 < at.rows ? __ldg(at.rs + (lane >> 2) + i * 8) : 1.0f;
+        rs[i] = row_scale && (lane >> 2) + i * 8 < at.rows ? at.rs[(lane >> 2) + i * 8] : 1.0f;
       ok = mbar_wait_cluster(&acc_full[acc], acc_phase, abort, status, 116);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
