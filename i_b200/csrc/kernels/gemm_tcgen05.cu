@@ -301,6 +301,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
     }
   } else if (warp == 1) {
+    grid_dependency_wait();                  // the bounded waits below must not count the conversion's time
     if (lane == 0) {
       // The 16-bit instantiation serves bf16 and fp16 operands: only the descriptor differs.
       const uint32_t idesc = KIND == Kind::BF16 && f16_operands ? make_idesc_fmt(Fmt::F16, kBM, BN)
@@ -515,6 +516,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #endif
     }
   } else if (warp == 1) {
+    grid_dependency_wait();                  // the bounded waits below must not count the conversion's time
     if (lane == 0 && rank == 1) {
       // Relay: tells the issuing CTA that this CTA's half of a stage has landed.
       int stage = 0;

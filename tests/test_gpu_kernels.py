@@ -487,6 +487,20 @@ def test_contract_16_bit_operands_of_every_layout(lib, torch, batch, m, n, k, ak
     assert (np.abs(got - want) / size).max() <= tol
 
 
+@pytest.mark.parametrize("precision", [F16, BF16])
+@pytest.mark.parametrize("m,n,k", [(3, 5, 1 << 24), (264, 256, 1 << 17)])
+def test_contract_16_bit_behind_a_long_conversion(lib, torch, precision, m, n, k):
+    # Few, very long rows: the GEMM is resident long before its operands are converted.  Ones and powers of
+    # two, so that every product and sum is exact.
+    a, b = torch.ones(m, k, device="cuda"), torch.ones(n, k, device="cuda")
+    a *= 2.0 ** torch.arange(m, device="cuda").remainder(9)[:, None]
+    c = torch.full((m, n), float("nan"), device="cuda")
+    wb = lib.ib_contract_workspace_bytes(1, m, n, k, 1, 1, precision)
+    ws = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    ok(lib, lib.ib_contract(a.data_ptr(), b.data_ptr(), c.data_ptr(), 1, m, n, k, 1, 1, precision, ws.data_ptr(), wb, None))
+    assert torch.equal(c, a[:, :1] * k + torch.zeros(n, device="cuda"))
+
+
 @pytest.mark.parametrize("batch,m,n,k", [
     (1, 33, 31, 31), (1, 32, 32, 2048), (3, 70, 50, 515),        # the smallest tile, whole and cut along k
     (1, 8, 8000, 40), (8, 300, 300, 128),                        # the middle tiles
