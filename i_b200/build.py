@@ -8,9 +8,11 @@ static CUDA runtime, so the library loads on a machine without a GPU or driver
 """
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
@@ -87,24 +89,46 @@ def _compile(src, headers, verbose, obj_dir=None, extra=()):
     return obj, proc.stderr if verbose else ""
 
 
+def call_module(kind, torch_version, out_dir=OUT_DIR):
+    """Path of the extension module `_<kind>_call` for this Python and, for "cuda", the given torch: a file
+    compiled against others is not found instead of misread."""
+    built_for = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
+    if kind == "cuda":
+        built_for = ".torch-%s%s" % (torch_version, built_for)
+    return os.path.join(out_dir, "_%s_call%s" % (kind, built_for))
+
+
+def _torch_version(torch_dir):
+    """torch.__version__, without importing torch."""
+    with open(os.path.join(torch_dir, "version.py")) as f:
+        return re.search(r"^__version__\s*=\s*['\"]([^'\"]+)", f.read(), re.M).group(1)
+
+
 def _build_call_modules(out_dir):
     """The extension modules ilang.py marshals its calls through (csrc/python): NumPy arrays with
-    Python's C API alone, CUDA tensors with torch's headers and libraries."""
-    import sysconfig
+    Python's C API alone, CUDA tensors with torch's headers and libraries.  Without what they are compiled
+    against they are left out: ilang.py then makes the same calls through ctypes."""
+    include = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write("i_b200.build: no Python.h in %s, calls go through ctypes\n" % include)
+        return
     common = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-I", os.path.join(REPO, "include"),
-              "-isystem", sysconfig.get_paths()["include"]]
-    jobs = {"host_call": []}
+              "-isystem", include]
+    jobs = {"host": (call_module("host", None, out_dir), [])}
     spec = importlib.util.find_spec("torch")
     if spec is not None and spec.submodule_search_locations:
         torch_dir = list(spec.submodule_search_locations)[0]
         inc, lib = os.path.join(torch_dir, "include"), os.path.join(torch_dir, "lib")
         cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(_nvcc()) or _nvcc()))),
                             "include")
-        jobs["cuda_call"] = ["-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
-                             "-isystem", cuda, "-L", lib, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    for name, extra in jobs.items():
-        src = os.path.join(CSRC, "python", name + ".cc")
-        out = os.path.join(out_dir, "_%s.so" % name)
+        if os.path.exists(os.path.join(lib, "libc10_cuda.so")) and os.path.isdir(os.path.join(inc, "c10")):
+            jobs["cuda"] = (call_module("cuda", _torch_version(torch_dir), out_dir),
+                            ["-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
+                             "-isystem", cuda, "-L", lib, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+        else:
+            sys.stderr.write("i_b200.build: torch in %s has no CUDA, its calls go through ctypes\n" % torch_dir)
+    for kind, (out, extra) in jobs.items():
+        src = os.path.join(CSRC, "python", kind + "_call.cc")
         if _newer(out, [src] + _headers()):
             continue
         proc = subprocess.run(common + [src, "-o", out] + extra, capture_output=True, text=True)

@@ -114,23 +114,28 @@ def set_reserved_sms(n):
 
 
 # Native marshalling of the common calls (csrc/python): the module that takes CUDA tensors, the one
-# that takes NumPy arrays; None until torch (NumPy) is in the process, False where there is none.
+# that takes NumPy arrays; None until torch (NumPy) is in the process, False where there is none that
+# fits this Python and this torch (calls then go through ctypes).
 _cuda_call = None
 _host_call = None
 
 
 def _load_call(kind, needs):
     """The extension module `_<kind>_call`, bound to the loaded library; None while the package it
-    `needs` is not in the process, False if it was not built."""
+    `needs` is not in the process, False if it was not built for these versions or does not load."""
     if needs not in sys.modules:
         return None
+    from . import build
     name = "_%s_call" % kind
-    path = os.path.join(_HERE, "lib", name + ".so")
+    path = build.call_module(kind, getattr(sys.modules[needs], "__version__", ""))
     if not os.path.exists(path):
         return False
     loader = importlib.machinery.ExtensionFileLoader(name, path)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
-    loader.exec_module(module)
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
+        loader.exec_module(module)
+    except ImportError:
+        return False
     symbols = ["i_b200_exec_into" if kind == "cuda" else "i_exec_into", "i_output_count",
                "i_output_ranks", "i_output_shapes", "i_error"]
     addresses = [ctypes.cast(getattr(_core, s), _VOIDP).value for s in symbols]

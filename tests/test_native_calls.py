@@ -1,5 +1,7 @@
 """The native call modules (i_b200/csrc/python) and the general route beside them: what the modules do not
 handle has to reach the general route, which words the errors, and nothing torch throws may end the process."""
+import importlib.machinery
+import os
 import subprocess
 import sys
 import textwrap
@@ -50,6 +52,36 @@ def test_tensors_without_memory_raise(ilang):
     run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=600)
     raised = [line.split()[0] for line in run.stdout.splitlines() if line.endswith(" raised")]
     assert run.returncode == 0 and raised == list(WRAPPERS), run.stdout[-500:] + run.stderr[-2000:]
+
+
+def test_modules_are_those_of_this_python_and_torch(ilang, monkeypatch, tmp_path):
+    # A module of another torch is not found; a file that does not load leaves the ctypes route.
+    from i_b200 import build
+    torch = pytest.importorskip("torch")
+    assert torch.__version__ in build.call_module("cuda", torch.__version__)
+    assert os.path.exists(build.call_module("cuda", torch.__version__))
+    assert ilang._load_call("cuda", "torch") and ilang._load_call("host", "numpy")
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0.1")
+        assert ilang._load_call("cuda", "torch") is False
+    broken = tmp_path / "broken.so"
+    broken.write_bytes(b"no library")
+    monkeypatch.setattr(build, "call_module", lambda *given: str(broken))
+    assert ilang._load_call("cuda", "torch") is False and ilang._load_call("host", "numpy") is False
+
+
+def test_the_build_does_without_what_the_modules_need(monkeypatch, tmp_path):
+    from i_b200 import build
+    no_cuda = tmp_path / "torch"
+    (no_cuda / "lib").mkdir(parents=True)
+    spec = importlib.machinery.ModuleSpec("torch", None, is_package=True)
+    spec.submodule_search_locations = [str(no_cuda)]
+    with monkeypatch.context() as m:
+        m.setattr(build.importlib.util, "find_spec", lambda name: spec)
+        m.setattr(build.subprocess, "run", lambda cmd, **_: subprocess.CompletedProcess(cmd, "cuda_call" in " ".join(cmd), "", ""))
+        build._build_call_modules(str(tmp_path))
+    monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    build._build_call_modules(str(tmp_path))
 
 
 @pytest.fixture
