@@ -17,6 +17,8 @@
 // (97 launches), here in one launch; figures in the table of the dispatch rule (dispatch.cu).
 #include <cooperative_groups.h>
 
+#include <cmath>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -415,6 +417,28 @@ bool attention_direct_shape_ok(size_t batch, size_t nq, size_t nk, size_t d, siz
   if (nk > (static_cast<size_t>(1) << 35)) return false;                 // blocks per split are an int
   return batch <= (static_cast<size_t>(1) << 24) && nq <= (static_cast<size_t>(1) << 24) &&
          batch * nq <= (static_cast<size_t>(1) << 27);                   // CTAs are a 31-bit grid
+}
+
+// Estimated time.  A CTA takes about as long with one warp busy (32 keys or fewer) as with all eight (256
+// keys), so the time is the number of rounds of CTAs, times the blocks of keys a warp takes in turn, times
+// what a block takes for so many queries and features; the last round counts in full.
+double attention_direct_us(size_t batch, size_t nq, size_t nk, size_t d, size_t dv) {
+  const DirectPlan p = direct_plan(batch, nq, nk);
+  const size_t widest = d > dv ? d : dv, features = widest <= 32 ? 32 : widest <= 64 ? 64 : 128;
+  const size_t room = static_cast<size_t>(kNumSMs) * (p.nq_per_cta >= 4 ? 2 : 3);
+  const size_t rounds = (batch * p.groups * static_cast<size_t>(p.splits) + room - 1) / room;
+  const size_t blocks = (static_cast<size_t>(p.blocks_per_split) + kWarps - 1) / kWarps;
+  return 2.0 + static_cast<double>(rounds * blocks) *
+                   (1.5 + 0.55 * p.nq_per_cta + (0.04 + 0.004 * p.nq_per_cta) * static_cast<double>(features));
+}
+
+// Whether the last round of CTAs leaves much of the machine idle, where there are too many heads to divide
+// their keys evenly.
+bool attention_direct_idles(size_t batch, size_t nq, size_t nk) {
+  const DirectPlan p = direct_plan(batch, nq, nk);
+  const double room = kNumSMs * (p.nq_per_cta >= 4 ? 2.0 : 3.0);
+  const double units = static_cast<double>(batch * p.groups), ctas = units * p.splits;
+  return units * 3.0 > room && ctas < (p.splits > 1 ? 0.7 : 0.6) * room * std::ceil(ctas / room);
 }
 
 size_t attention_direct_floats(size_t batch, size_t nq, size_t nk, size_t dv) {

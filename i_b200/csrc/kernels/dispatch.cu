@@ -83,17 +83,31 @@ bool attention_shape_ok(size_t d, size_t dv) {
 //   up to kDirectQueries queries per head, under every precision: the pass is then bound by reading K
 //   and V once, which the tensor arms cannot do (they first write converted copies of both, as many
 //   bytes again), and no arm is less exact.  32 heads x 10000 keys x 128 on B200, direct / fp16 arm /
-//   bf16 arm: 4 queries 80 / 207 / 135 us, 8 queries 115 / 207 / 136, 16 queries 204 / 210 / 139;
+//   bf16 arm: 4 queries 80 / 207 / 135 us, 8 queries 115 / 207 / 136, 16 queries 204 / 210 / 139.  The bf16
+//   arm is ahead for five to eight queries of a number of heads that fills the last round badly (direct /
+//   bf16, 8 x 4000 x 128: 148 heads 179 / 222, 160 heads 321 / 261, 300 heads 548 / 464), unless the keys
+//   are so few that its launches count (200 heads x 8 x 200 x 128: 26 / 31);
 //   otherwise fp32 arithmetic up to kDirectFlop: above, two tiled contractions with the scores in
 //   memory between them are faster (8 x 256 x 256 x 64, 2^27: 17.6 / 19.7 us; 1024 x 1024 x 64, 2^28:
 //   30.6 / 26.8).
+// In fp32 few keys for many queries go to the contractions too: 32 keys give one of a CTA's eight warps
+// work, and rounds of such CTAs take longer than the three launches.  Direct / contractions: 16384 x 16 x 64
+// 75 / 19 us, 64 heads x 256 x 16 x 64 76 / 19, 2000 x 16 x 16 x 32 105 / 25, 8000 x 4 x 32 x 32 144 / 59;
+// 600 x 32 x 64 12.4 / 14.5, 64 x 30 x 30 x 30 14.4 / 16.5.  The line is where the estimates meet, up to 512 keys
+// (of 220 shapes the slower form is taken in nine, by at most 13 %).  The contractions' tiles are 32 wide.
 constexpr size_t kDirectQueries = 8;
 constexpr double kDirectFlop = 134217728.0;     // 2^27
 bool attention_prefers_direct(size_t batch, size_t nq, size_t nk, size_t d, size_t dv, bool v_kmajor, int precision) {
   if (v_kmajor || !attention_direct_shape_ok(batch, nq, nk, d, dv)) return false;
-  if (nq <= kDirectQueries) return true;
   const double flop = 4.0 * batch * nq * nk * d;
-  return !wants_tensor(precision, flop) && flop <= kDirectFlop;
+  const bool tensor = wants_tensor(precision, flop);
+  if (nq <= kDirectQueries && (tensor || nk > 256))
+    return precision != IB_PRECISION_BF16 || nq <= 4 || nk <= 512 || !attention_shape_ok(d, dv) ||
+           !attention_direct_idles(batch, nq, nk);
+  if (tensor || (nq > kDirectQueries && flop > kDirectFlop)) return false;
+  if (nk > 512) return true;
+  const double tiles_flop = 4.0 * batch * round_up(nq, 32) * round_up(nk, 32) * d;
+  return attention_direct_us(batch, nq, nk, d, dv) <= 15.0 + (nk > 32 ? 1.5 : 0.0) + tiles_flop / 24e6;
 }
 
 // Which arithmetic the fused attention kernel uses for a precision request: AUTO and F16 take the

@@ -170,6 +170,8 @@ int prepare_attention_operands_bf16(const float* k, void* k16, const float* v, v
 // few queries per head or small problems.  `partials` holds attention_direct_floats floats (8-byte
 // aligned; null when that is 0).
 bool attention_direct_shape_ok(size_t batch, size_t nq, size_t nk, size_t d, size_t dv);
+double attention_direct_us(size_t batch, size_t nq, size_t nk, size_t d, size_t dv);   // an estimate
+bool attention_direct_idles(size_t batch, size_t nq, size_t nk);
 size_t attention_direct_floats(size_t batch, size_t nq, size_t nk, size_t dv);
 int attention_direct(const float* q, const float* k, const float* v, float* o, size_t batch, size_t nq,
                      size_t nk, size_t d, size_t dv, const float* logit_scale, bool logit_divide,

@@ -1034,6 +1034,29 @@ def test_attention_direct_fp32(lib, torch, batch, nq, nk, d, dv, scale):
     assert max_rel_to_peak(out.cpu().numpy(), want) <= TOL_FP32
 
 
+@pytest.mark.parametrize("batch,nq,nk,d,precision,tol,direct", [
+    (1, 600, 32, 64, FP32, 1e-5, True), (1, 9600, 32, 64, FP32, 1e-5, False),     # few keys: one warp of eight is busy
+    (1, 9601, 9, 33, FP32, 1e-5, False), (64, 30, 30, 30, FP32, 1e-5, True), (66, 4, 64, 128, FP32, 1e-5, True),
+    (8000, 4, 32, 32, FP32, 1e-5, False), (500, 1, 200, 32, FP32, 1e-5, True), (32, 8, 400, 64, FP32, 1e-5, True),
+    (148, 8, 1000, 64, BF16, TOL_BF16, True), (160, 8, 1000, 64, BF16, TOL_BF16, False),   # a last round of twelve heads
+    (160, 8, 1000, 64, F16, TOL_TF32, True), (160, 4, 1000, 64, BF16, TOL_BF16, True)])
+def test_attention_goes_direct_where_that_is_faster(lib, torch, batch, nq, nk, d, precision, tol, direct):
+    # Either side of the rule: one launch, or a merge of key ranges besides; the other routes take three or more.
+    g = torch.Generator(device="cuda")
+    g.manual_seed(batch + nq + nk)
+    q = torch.randn(batch, nq, d, device="cuda", generator=g) * d ** -0.5
+    k, v = (torch.randn(batch, nk, d, device="cuda", generator=g) for _ in range(2))
+    ws_bytes = lib.ib_attention_workspace_bytes(batch, nq, nk, d, d, 0, precision)
+    ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device="cuda")
+    o = torch.full((batch, nq, d), float("nan"), device="cuda")
+    before = lib.i_b200_launch_count()
+    ok(lib, lib.ib_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), batch, nq, nk, d, d, 0,
+                             precision, 0, ws.data_ptr(), ws_bytes, None))
+    assert (lib.i_b200_launch_count() - before == 1) == direct
+    want = torch.softmax(q.double() @ k.double().transpose(1, 2), -1) @ v.double()
+    assert ((o.double() - want).abs().max() / want.abs().max()).item() <= tol
+
+
 @pytest.mark.parametrize("precision,tol", [(F16, TOL_TF32), (BF16, TOL_BF16), (TF32_F16, TOL_TF32), (TF32, TOL_TF32)])
 @pytest.mark.parametrize("batch,nq,nk,d,divided", [
     (1, 2048, 2048, 128, (TF32_F16, TF32)),             # sixteen row tiles of sixteen key tiles
