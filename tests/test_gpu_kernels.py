@@ -516,6 +516,47 @@ def test_contract_fp32_tiles_and_parts(lib, torch, batch, m, n, k, akm, bkm):
     assert max_rel_to_peak(np.asarray(got).reshape(want.shape), want) <= TOL_FP32
 
 
+ADD, MUL, SUB, MAX, MIN = 0, 1, 2, 4, 5
+
+
+@pytest.mark.parametrize("batch,m,n,k", [
+    (1, 33, 31, 31), (1, 32, 32, 2048), (3, 70, 52, 515), (2, 5, 3, 700),       # the smallest tile, whole and cut along k
+    (1, 8, 8000, 40), (8, 300, 300, 128), (2000, 33, 33, 8),                    # the middle tiles
+    (1, 1000, 1030, 9), (1, 1920, 2049, 129), (1, 2050, 2052, 16)])             # the large ones
+@pytest.mark.parametrize("ops,modes", [
+    # (operator, left, right): the running value once; modes of the operands 0, 1, 2.
+    (((ADD, PREV, 0), (SUB, 1, PREV), (MUL, PREV, 2), (MAX, 0, PREV), (MIN, PREV, NONE), (SUB, PREV, NONE)), (2, 0, 1)),
+    (((MUL, PREV, 0), (MIN, 1, PREV), (ADD, PREV, NONE), (SUB, PREV, 2), (MAX, PREV, NONE)), (0, 3, 2)),
+    (((MUL, PREV, NONE), (SUB, 0, PREV), (MAX, PREV, 1)), (1, 3))])
+def test_contract_fp32_operators_on_every_tile(lib, torch, batch, m, n, k, ops, modes):
+    # Bit for bit the contraction followed by the pointwise kernel: same arithmetic, operator by operator.
+    vp, sz, ci = ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int
+    pi, pp = ctypes.POINTER(ci), ctypes.POINTER(vp)
+    lib.ib_contract_chain.argtypes = [vp, vp, vp, sz, sz, sz, sz, ci, ci, ci, sz, sz, ci, pi, ci, pp, pi, vp, sz, vp]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + n + k)
+    rows = batch * m
+    shapes = {0: (rows, n), 1: (rows,), 2: (n,), 3: ()}
+    operands = [torch.randn(shapes[mode], device="cuda", generator=g) for mode in modes]
+    a, b = torch.randn(batch, m, k, device="cuda", generator=g), torch.randn(batch, n, k, device="cuda", generator=g)
+    wb = lib.ib_contract_workspace_bytes(batch, m, n, k, 1, 1, FP32)
+    ws = torch.empty(max(wb, 256), dtype=torch.uint8, device="cuda")
+    plain, got = (torch.full((rows, n), float("nan"), device="cuda") for _ in range(2))
+    flat = [x for op in ops for x in op]
+    ok(lib, lib.ib_contract_chain(a.data_ptr(), b.data_ptr(), got.data_ptr(), batch, m, n, k, 1, 1, FP32, 0, 0, len(ops),
+                                  (ci * len(flat))(*flat), len(modes), (vp * len(modes))(*(x.data_ptr() for x in operands)),
+                                  (ci * len(modes))(*modes), ws.data_ptr(), wb, None))
+    ok(lib, lib.ib_contract(a.data_ptr(), b.data_ptr(), plain.data_ptr(), batch, m, n, k, 1, 1, FP32, ws.data_ptr(), wb, None))
+    # As an ib_map_chain call: the contraction's result is operand 0 and starts the chain.
+    code = [[op] + [(0 if j == 0 else PREV) if x == PREV else NONE if x == NONE else x + 1 for x in sides]
+            for j, (op, *sides) in enumerate(ops)]
+    flat = [x for op in code for x in op]
+    listed = [plain] + operands
+    ok(lib, lib.ib_map_chain(len(ops), (ci * len(flat))(*flat), len(listed), (vp * len(listed))(*(x.data_ptr() for x in listed)),
+                             (ci * len(listed))(0, *modes), plain.data_ptr(), rows, n, None))
+    assert torch.equal(got, plain)
+
+
 @pytest.mark.parametrize("m,n,k,akm,bkm", [
     (8, 7, 16, True, False),      # ilang-python/test.py:40-59
     (100, 40, 33, True, True), (65, 130, 17, False, True), (64, 64, 64, False, False),
