@@ -797,7 +797,8 @@ __device__ __forceinline__ void prepare_strip(const ContractOperand& o, unsigned
   if (SCALED && parts > 1) cg::this_cluster().sync();      // nobody leaves while its maxima are read
 }
 
-template <bool SCALED, int TPR>
+// SHORT: rows of at most TPR quads.
+template <bool SCALED, int TPR, bool SHORT>
 __global__ void __launch_bounds__(256)
 prepare_contract_kernel(const ContractOperand a, const ContractOperand b, size_t batch, size_t k, size_t kp,
                         unsigned parts) {
@@ -815,56 +816,94 @@ prepare_contract_kernel(const ContractOperand a, const ContractOperand b, size_t
   const size_t quads = kp / 4, rows = batch * o.rows;
   const unsigned at = threadIdx.x % TPR;
   const bool vec = k % 4 == 0 && (reinterpret_cast<uintptr_t>(o.in) & 15u) == 0;
-  const bool held = quads <= TPR * 8;
   constexpr unsigned kGroups = 256 / TPR;
-  for (size_t r0 = static_cast<size_t>(block) * kGroups; r0 < rows; r0 += static_cast<size_t>(o.blocks) * kGroups) {
-    const size_t r = r0 + threadIdx.x / TPR;
-    const bool live = r < rows;
-    const float* src = o.in + r * k;
-    uint16_t* dst = static_cast<uint16_t*>(o.out) + r * kp;
-    float4 x[8];
-    auto fetch = [&](size_t q0) {
+  if constexpr (SHORT) {
+    // A quad a thread and row: eight rows at a time, so that as many loads are in flight.
+    const size_t c = at * 4;
+    for (size_t r0 = static_cast<size_t>(block) * kGroups * 8; r0 < rows; r0 += static_cast<size_t>(o.blocks) * kGroups * 8) {
+      float4 x[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const size_t c = (q0 + u * TPR) * 4;
+        const size_t r = r0 + u * kGroups + threadIdx.x / TPR;
         x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (live && vec && c < k) {
-          x[u] = __ldg(reinterpret_cast<const float4*>(src + c));
-        } else if (live && c < k) {
-          x[u].x = src[c];
-          if (c + 1 < k) x[u].y = src[c + 1];
-          if (c + 2 < k) x[u].z = src[c + 2];
-          if (c + 3 < k) x[u].w = src[c + 3];
+        if (r >= rows || c >= k) continue;
+        const float* src = o.in + r * k + c;
+        if (vec) {
+          x[u] = __ldg(reinterpret_cast<const float4*>(src));
+        } else {
+          x[u].x = src[0];
+          if (c + 1 < k) x[u].y = src[1];
+          if (c + 2 < k) x[u].z = src[2];
+          if (c + 3 < k) x[u].w = src[3];
         }
       }
-    };
-    float inv = 1.0f;
-    if (SCALED) {
-      float m = 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const size_t r = r0 + u * kGroups + threadIdx.x / TPR;
+        float inv = 1.0f;
+        if (SCALED) {
+          float m = fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w)));
+#pragma unroll
+          for (int d = TPR / 2; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+          const float scale = f16_scale_for(m);
+          inv = 1.0f / scale;
+          if (at == 0 && r < rows) o.scale[r] = scale;
+        }
+        if (r < rows && at < quads)
+          *reinterpret_cast<uint2*>(static_cast<uint16_t*>(o.out) + r * kp + c) = pack4_16<SCALED>(x[u], inv);
+      }
+    }
+  } else {
+    const bool held = quads <= TPR * 8;
+    for (size_t r0 = static_cast<size_t>(block) * kGroups; r0 < rows; r0 += static_cast<size_t>(o.blocks) * kGroups) {
+      const size_t r = r0 + threadIdx.x / TPR;
+      const bool live = r < rows;
+      const float* src = o.in + r * k;
+      uint16_t* dst = static_cast<uint16_t*>(o.out) + r * kp;
+      float4 x[8];
+      auto fetch = [&](size_t q0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const size_t c = (q0 + u * TPR) * 4;
+          x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (live && vec && c < k) {
+            x[u] = __ldg(reinterpret_cast<const float4*>(src + c));
+          } else if (live && c < k) {
+            x[u].x = src[c];
+            if (c + 1 < k) x[u].y = src[c + 1];
+            if (c + 2 < k) x[u].z = src[c + 2];
+            if (c + 3 < k) x[u].w = src[c + 3];
+          }
+        }
+      };
+      float inv = 1.0f;
+      if (SCALED) {
+        float m = 0.0f;
+        for (size_t q0 = at; q0 < quads; q0 += TPR * 8) {
+          fetch(q0);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
+        }
+        m = warp_fold<IB_OP_MAX>(m);
+        if (TPR > 32) {
+          __syncthreads();                     // part_max may still be read for the rows before
+          if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = m;
+          __syncthreads();
+#pragma unroll
+          for (int w = 0; w < TPR / 32; ++w) m = fmaxf(m, part_max[threadIdx.x / TPR * (TPR / 32) + w]);
+        }
+        const float scale = f16_scale_for(m);
+        inv = 1.0f / scale;
+        if (at == 0 && live) o.scale[r] = scale;
+      }
       for (size_t q0 = at; q0 < quads; q0 += TPR * 8) {
-        fetch(q0);
+        if (!SCALED || !held) fetch(q0);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-          m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
+          if (live && q0 + u * TPR < quads)
+            *reinterpret_cast<uint2*>(dst + (q0 + u * TPR) * 4) = pack4_16<SCALED>(x[u], inv);
       }
-      m = warp_fold<IB_OP_MAX>(m);
-      if (TPR > 32) {
-        __syncthreads();                     // part_max may still be read for the rows before
-        if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = m;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < TPR / 32; ++w) m = fmaxf(m, part_max[threadIdx.x / TPR * (TPR / 32) + w]);
-      }
-      const float scale = f16_scale_for(m);
-      inv = 1.0f / scale;
-      if (at == 0 && live) o.scale[r] = scale;
-    }
-    for (size_t q0 = at; q0 < quads; q0 += TPR * 8) {
-      if (!SCALED || !held) fetch(q0);
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (live && q0 + u * TPR < quads)
-          *reinterpret_cast<uint2*>(dst + (q0 + u * TPR) * 4) = pack4_16<SCALED>(x[u], inv);
     }
   }
 }
@@ -990,8 +1029,10 @@ int prepare_contract_operands(const float* a, bool a_kmajor, void* a16, float* a
   if (batch == 0 || m == 0 || n == 0 || k == 0) return 0;
   const bool scaled = a_scale != nullptr;
   // As few threads a row as hold it (32 values each): the more loads a thread has in flight, the less the
-  // wait for the row's maximum shows.
-  const int tpr = kp <= 1024 ? 32 : kp <= 2048 ? 64 : kp <= 4096 ? 128 : 256;
+  // wait for the row's maximum shows.  Rows of up to 128 values take a thread a quad, eight rows at a time:
+  // with a warp a row and one load a thread, 9 x 4048 rows of 29 took 14.5 us, 10^6 rows of 24 260.
+  const int tpr = kp <= 32 ? 8 : kp <= 64 ? 16 : kp <= 1024 ? 32 : kp <= 2048 ? 64 : kp <= 4096 ? 128 : 256;
+  const size_t at_once = kp <= 128 ? 8 : 1;
   // A strip's k range is divided until there are about two CTAs an SM or a part has 128 lines left.
   auto strips = [&](size_t rows, bool kmajor) { return kmajor ? 0 : batch * ((rows + 31) / 32); };
   const size_t n_strips = strips(m, a_kmajor) + strips(n, b_kmajor);
@@ -999,7 +1040,8 @@ int prepare_contract_operands(const float* a, bool a_kmajor, void* a16, float* a
   while (n_strips && parts < 8 && n_strips * parts < 2 * static_cast<size_t>(kNumSMs) && kp / (parts * 2) >= kStripK)
     parts *= 2;
   auto blocks_for = [&](size_t rows, bool kmajor) {
-    const size_t blocks = kmajor ? std::min((batch * rows * tpr + 255) / 256, static_cast<size_t>(kNumSMs) * 32)
+    const size_t blocks = kmajor ? std::min((batch * rows * tpr + 256 * at_once - 1) / (256 * at_once),
+                                            static_cast<size_t>(kNumSMs) * 32)
                                  : strips(rows, kmajor) * parts;
     return (blocks + parts - 1) / parts * parts;            // a cluster serves one operand
   };
@@ -1017,12 +1059,15 @@ int prepare_contract_operands(const float* a, bool a_kmajor, void* a16, float* a
   cfg.stream = s;
   cfg.attrs = &cluster;
   cfg.numAttrs = parts > 1 ? 1 : 0;
-  auto pick = [tpr](auto is_scaled) {
+  auto pick = [tpr, at_once](auto is_scaled) {
     constexpr bool kScaled = decltype(is_scaled)::value;
-    return tpr == 32   ? &prepare_contract_kernel<kScaled, 32>
-           : tpr == 64  ? &prepare_contract_kernel<kScaled, 64>
-           : tpr == 128 ? &prepare_contract_kernel<kScaled, 128>
-                        : &prepare_contract_kernel<kScaled, 256>;
+    return tpr == 8    ? &prepare_contract_kernel<kScaled, 8, true>
+           : tpr == 16  ? &prepare_contract_kernel<kScaled, 16, true>
+           : at_once > 1 ? &prepare_contract_kernel<kScaled, 32, true>
+           : tpr == 32  ? &prepare_contract_kernel<kScaled, 32, false>
+           : tpr == 64  ? &prepare_contract_kernel<kScaled, 64, false>
+           : tpr == 128 ? &prepare_contract_kernel<kScaled, 128, false>
+                        : &prepare_contract_kernel<kScaled, 256, false>;
   };
   auto* kernel = scaled ? pick(std::true_type{}) : pick(std::false_type{});
   if (cudaLaunchKernelEx(&cfg, kernel, oa, ob, batch, k, kp, parts) != cudaSuccess)

@@ -487,6 +487,14 @@ def test_contract_16_bit_operands_of_every_layout(lib, torch, batch, m, n, k, ak
     assert (np.abs(got - want) / size).max() <= tol
 
 
+@pytest.mark.parametrize("batch,m,n,k", [(3, 70, 300, 1), (1, 9, 2000, 24), (2, 40, 131, 29), (1, 300, 33, 64),
+                                         (1, 33, 70, 65), (2, 131, 9, 128), (1, 100, 101, 129)])   # 8, 16, 32 threads a row
+@pytest.mark.parametrize("akm,bkm", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("precision,tol", [(F16, 1e-3), (BF16, 8e-3)])
+def test_contract_16_bit_operands_of_short_rows(lib, torch, batch, m, n, k, akm, bkm, precision, tol):
+    test_contract_16_bit_operands_of_every_layout(lib, torch, batch, m, n, k, akm, bkm, precision, tol)
+
+
 @pytest.mark.parametrize("precision", [F16, BF16])
 @pytest.mark.parametrize("m,n,k", [(3, 5, 1 << 24), (264, 256, 1 << 17)])
 def test_contract_16_bit_behind_a_long_conversion(lib, torch, precision, m, n, k):
