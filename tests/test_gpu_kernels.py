@@ -495,6 +495,22 @@ def test_contract_16_bit_operands_of_short_rows(lib, torch, batch, m, n, k, akm,
     test_contract_16_bit_operands_of_every_layout(lib, torch, batch, m, n, k, akm, bkm, precision, tol)
 
 
+@pytest.mark.parametrize("batch,m,n,k", [(1, 5, 3000, 24), (1, 3000, 5, 24), (2, 9, 33, 40), (1, 33, 257, 16),
+                                         (3, 161, 1, 64), (1, 129, 260, 8), (1, 290, 258, 32)])
+@pytest.mark.parametrize("precision,tol", [(TF32, 2e-3), (F16, 1e-3), (BF16, 8e-3)])
+def test_contract_results_of_few_rows_or_columns(lib, torch, batch, m, n, k, precision, tol):
+    # Warps without a row, chunks without a column; nothing is written beside the result.
+    a, b = (torch.randn(batch, r, k, device="cuda") for r in (m, n))
+    out = torch.full((batch * m * n + 64,), float("nan"), device="cuda")
+    wb = lib.ib_contract_workspace_bytes(batch, m, n, k, 1, 1, precision)
+    ws = torch.empty(max(wb, 256), dtype=torch.uint8, device="cuda")
+    ok(lib, lib.ib_contract(a.data_ptr(), b.data_ptr(), out.data_ptr(), batch, m, n, k, 1, 1, precision, ws.data_ptr(), wb, None))
+    want = a.double() @ b.double().transpose(1, 2)
+    size = a.double().norm(dim=2)[:, :, None] * b.double().norm(dim=2)[:, None, :]
+    assert ((out[:-64].view(batch, m, n).double() - want).abs() / size).max().item() <= tol
+    assert torch.isnan(out[-64:]).all()
+
+
 @pytest.mark.parametrize("precision", [F16, BF16])
 @pytest.mark.parametrize("m,n,k", [(3, 5, 1 << 24), (264, 256, 1 << 17)])
 def test_contract_16_bit_behind_a_long_conversion(lib, torch, precision, m, n, k):
