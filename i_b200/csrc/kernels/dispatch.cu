@@ -426,6 +426,13 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
     const bool a_rows = !dots && n == 1 && a_kmajor != 0;     // C[b][i] = A[b][i][:] . B[b][:]
     const bool b_rows = !dots && m == 1 && b_kmajor != 0;     // C[b][j] = A[b][:] . B[b][j][:]
     constexpr size_t kMostLaunches = 64;
+    // Operators run in the fold's last step where that saves a launch and lengthens one fold only a little: one
+    // batch entry, and rows few enough that the one lane a row that applies them is not the longer part (with
+    // a full-size operand, fused / apart in us: 4096 x 4096 14.5 / 16.5, 10000 x 200 8.3 / 10.4, 20000 x 2000
+    // 39.7 / 38.3, 200000 x 20 46.6 / 28.9; 8 entries of 1000 x 100 49 / 37).  Down the columns a thread has
+    // a column each.
+    constexpr size_t kFusedRows = 12000;
+    const bool rows_fused = batch == 1 && n <= kFusedRows;
     if (dots || ((a_rows || b_rows) && batch <= kMostLaunches)) {
       int rc = 0;
       if (dots) {
@@ -434,14 +441,14 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
                                   (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0
                               ? static_cast<float*>(workspace)
                               : nullptr;
-        rc = dot_rows(a, b, false, c, batch, k, s, partials, fused);
+        rc = dot_rows(a, b, false, c, batch, k, s, partials, batch <= kFusedRows ? fused : nullptr);
       } else {
         const size_t rows = a_rows ? m : n;
         for (size_t e = 0; e < batch && rc == 0; ++e)
           rc = dot_rows((a_rows ? a : b) + e * rows * k, (a_rows ? b : a) + e * k, true, c + e * rows,
-                        rows, k, s, nullptr, b_rows ? fused : nullptr, e);
+                        rows, k, s, nullptr, b_rows && rows_fused ? fused : nullptr, e);
       }
-      return b_rows || dots ? rc : then_chain(rc);
+      return (dots && batch <= kFusedRows) || (b_rows && rows_fused) ? rc : then_chain(rc);
     }
     // The same with the matrix stored k-major the other way round, [k][rows]: vector times
     // matrix, a weighted fold down the columns.
@@ -457,8 +464,8 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
       int rc = 0;
       for (size_t e = 0; e < batch && rc == 0; ++e)
         rc = dot_leading_axis((a_cols ? a : b) + e * k * cols, (a_cols ? b : a) + e * k, c + e * cols, k,
-                              cols, partials, s, b_cols ? fused : nullptr, e);
-      return b_cols ? rc : then_chain(rc);
+                              cols, partials, s, b_cols && batch == 1 ? fused : nullptr, e);
+      return b_cols && batch == 1 ? rc : then_chain(rc);
     }
   }
   const double flop = 2.0 * batch * m * n * k;

@@ -611,5 +611,11 @@ def test_operators_on_a_matrix_vector_product(ilang, k):
     m, s = rand((3, 20, k), 74), rand((3, k), 75)
     plain = i("bij*bj~bij") >> i("+bij~bi")
     shifted = plain >> i("bi+b~bi") >> i("bi*i~bi")
+    # Rows too many for the fold's last step, and one batch entry of few.
+    tall, v, shift = rand((12001, 9), 78), rand((9,), 79), rand((12001,), 80)
+    plain_rows = i("j*ij~ij") >> i("+ij~i")
+    for n in (12000, 12001):
+        got = (plain_rows >> i("i+i~i") >> i(">i~i")).exec_numpy(v, tall[:n], shift[:n])
+        assert np.array_equal(got, np.maximum(plain_rows.exec_numpy(v, tall[:n]) + shift[:n], 0))
     c, w = rand((3,), 76), rand((20,), 77)
     assert np.array_equal(shifted.exec_numpy(m, s, c, w), (plain.exec_numpy(m, s) + c[:, None]) * w[None, :])
