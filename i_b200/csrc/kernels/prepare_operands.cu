@@ -593,33 +593,31 @@ prepare_attention_mixed_kernel(PrepareMixedArgs a) {
   prepare_v_f16_by_quarters(a, tile, scratch);
 }
 
-// fp16 arm.  blockIdx.y = 0: K, one tile of 128 keys per block at a time: the tile is read once
-// (twice, the second time from cache, without FEW_TILES), its largest magnitude decides the power of
-// two that brings it into [2^14, 2^15), and fp16(K / that) is written with rows padded to d_pitch (pad
-// columns zero).  An outlier key therefore costs precision only to the 127 keys beside it.
-// blockIdx.y = 1: the fp16 V^T as in the mixed arm.
+// fp16 arm.  K, one tile of 128 keys per block at a time: a thread keeps its share of the tile in registers
+// (sixteen 16-byte loads in flight), the tile's largest magnitude decides the power of two that brings it into
+// [2^14, 2^15), and fp16(K / that) is written with rows padded to d_pitch (pad columns zero).  An outlier
+// key therefore costs precision only to the 127 keys beside it.  V: the fp16 V^T as in the mixed arm.
+// HALVES: K and V in one grid (blockIdx.y picks), or either in a grid of its own, since the registers that
+// hold K's tile would leave the V half of a large grid two blocks per SM.
 // Bound by HBM.  A thread's place in the tile comes from shifts: with a division of 64-bit numbers
 // by the row length per 16-byte load the K half of 64 heads x 2048 x 128 took 35 us for 100 MB, now 21.
-template <bool FEW_TILES>
+enum class Halves { Both, K, V };
+template <Halves HALVES>
 __global__ void __launch_bounds__(256)
-prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
-  __shared__ uint32_t words[128][32];      // a step of V^T: 128 features x 32 key pairs (fp16x2)
+prepare_attention_f16_kernel(PrepareMixedArgs a) {
   __shared__ float scratch[8];
   sm100::trigger_dependent_launch();       // see prepare_attention_kernel
-  // halves: 3 = this grid does both (blockIdx.y picks), 1 = K only, 2 = V only.
-  if ((halves == 3 ? blockIdx.y : halves - 1) == 1) {
-    prepare_v_f16(a, words, scratch);
-    return;
+  if constexpr (HALVES != Halves::K) {
+    __shared__ uint32_t words[128][32];    // a step of V^T: 128 features x 32 key pairs (fp16x2)
+    if (HALVES == Halves::V || blockIdx.y == 1) {
+      prepare_v_f16(a, words, scratch);
+      return;
+    }
   }
   // 4-column groups per (padded) key row: at most 32, rounded up to a power of two.
   const unsigned across = 32 - __clz(static_cast<unsigned>(a.d_pitch / 4) - 1);
   const bool vec = (reinterpret_cast<uintptr_t>(a.k) & 15u) == 0;   // d is a multiple of 4
-  // With few tiles (one head of a few thousand keys) the blocks are too few to hide two rounds of
-  // loads each: a thread then keeps its share of the tile in registers (sixteen 16-byte loads in
-  // flight, 118 registers) and the second pass is free.  With many tiles that register count
-  // would hold the V half of this grid to two blocks per SM, and eight loads at a time at 64
-  // registers is the faster whole.
-  constexpr int kBatch = FEW_TILES ? 16 : 8;
+  constexpr int kBatch = 16;                 // 128 keys x 32 groups over 256 threads
   for (size_t t = blockIdx.x; t < a.batch * a.kv_tiles; t += gridDim.x) {
     const size_t b = t / a.kv_tiles, key0 = (t - b * a.kv_tiles) * 128;
     const size_t keys = a.nk - key0 < 128 ? a.nk - key0 : 128;
@@ -634,17 +632,13 @@ prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
       const float* at = src + r * static_cast<unsigned>(a.d) + c;
       return vec ? *reinterpret_cast<const float4*>(at) : make_float4(at[0], at[1], at[2], at[3]);
     };
-    // Pass 1: the tile's largest magnitude.  Pass 2 reads the same 64 KB again, from cache, unless
-    // the thread's whole share (128 x 32 groups over 256 threads = 16) is still in registers.
     float m = 0.0f;
     float4 x[kBatch];
-    for (unsigned g0 = threadIdx.x; g0 < places; g0 += 256 * kBatch) {
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) x[u] = fetch(g0 + u * 256);
+    for (int u = 0; u < kBatch; ++u) x[u] = fetch(threadIdx.x + u * 256);
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u)
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
-    }
+    for (int u = 0; u < kBatch; ++u)
+      m = fmaxf(m, fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w))));
     m = warp_fold<IB_OP_MAX>(m);
     __syncthreads();                         // scratch may still be read from the tile before
     if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
@@ -654,25 +648,19 @@ prepare_attention_f16_kernel(PrepareMixedArgs a, int halves) {
     const float scale = f16_scale_for(all);
     const float inv = 1.0f / scale;
     if (threadIdx.x == 0) a.k_tile_scale[t] = scale;
-    for (unsigned g0 = threadIdx.x; g0 < places; g0 += 256 * kBatch) {
-      if (!FEW_TILES) {
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) x[u] = fetch(g0 + u * 256);
-      }
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        const unsigned g = g0 + u * 256;
-        const unsigned r = g >> across, c = (g & ((1u << across) - 1)) * 4;
-        if (g < places && c < a.d_pitch) {
-          *reinterpret_cast<uint2*>(dst + r * static_cast<unsigned>(a.d_pitch) + c) =
-              pack4_f16(x[u].x * inv, x[u].y * inv, x[u].z * inv, x[u].w * inv);
-        }
+    for (int u = 0; u < kBatch; ++u) {
+      const unsigned g = threadIdx.x + u * 256;
+      const unsigned r = g >> across, c = (g & ((1u << across) - 1)) * 4;
+      if (g < places && c < a.d_pitch) {
+        *reinterpret_cast<uint2*>(dst + r * static_cast<unsigned>(a.d_pitch) + c) =
+            pack4_f16(x[u].x * inv, x[u].y * inv, x[u].z * inv, x[u].w * inv);
       }
     }
   }
   // Launched on its own under the tail of the maxima kernel (many tiles): this grid then only
   // completes once that one has, so that whoever waits for this grid has waited for both.
-  if (halves == 1) sm100::grid_dependency_wait();
+  if (HALVES == Halves::K) sm100::grid_dependency_wait();
 }
 
 // ---- operands of a contraction for the 16-bit tensor arms: both in one launch ----------------
@@ -990,21 +978,20 @@ int prepare_attention_operands_f16(const float* k, void* k16, float* k_tile_scal
   cfg.numAttrs = 1;
   cudaError_t launched;
   if (batch * kv_tiles <= 512) {
-    // Few tiles: one grid, both halves, K tiles held in registers.
+    // Few tiles: one grid, both halves.
     cfg.gridDim = dim3(static_cast<unsigned>(std::min(std::max(batch * kv_tiles, v_blocks), cap)), 2);
-    launched = cudaLaunchKernelEx(&cfg, prepare_attention_f16_kernel<true>, a, 3);
+    launched = cudaLaunchKernelEx(&cfg, prepare_attention_f16_kernel<Halves::Both>, a);
   } else {
-    // Many tiles: K with each tile held in registers (128 registers: in one grid with the V half
-    // it would halve that half's occupancy; with two passes per tile instead it measured 1.8x the
-    // bf16 conversion's time), running beside the maxima kernel, which it does not need but whose
+    // Many tiles: K in a grid of its own (with two passes per tile instead of the tile in registers, both in
+    // one grid, it measured 1.8x the bf16 conversion's time), running beside the maxima kernel, which it does not need but whose
     // completion it waits for before it ends; then V, which waits for the K grid and so for the
     // maxima.  The attention kernel that waits for the V grid thereby waits for all three.
     cfg.gridDim = dim3(static_cast<unsigned>(std::min(batch * kv_tiles, cap * 2)), 1);
-    launched = cudaLaunchKernelEx(&cfg, prepare_attention_f16_kernel<true>, a, 1);
+    launched = cudaLaunchKernelEx(&cfg, prepare_attention_f16_kernel<Halves::K>, a);
     if (launched == cudaSuccess) {
       count_launch();
       cfg.gridDim = dim3(static_cast<unsigned>(std::min(v_blocks, cap)), 1);
-      launched = cudaLaunchKernelEx(&cfg, prepare_attention_f16_kernel<false>, a, 2);
+      launched = cudaLaunchKernelEx(&cfg, prepare_attention_f16_kernel<Halves::V>, a);
     }
   }
   if (launched != cudaSuccess)
