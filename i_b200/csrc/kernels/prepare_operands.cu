@@ -790,7 +790,7 @@ template <bool SCALED, int TPR, bool SHORT>
 __global__ void __launch_bounds__(256)
 prepare_contract_kernel(const ContractOperand a, const ContractOperand b, size_t batch, size_t k, size_t kp,
                         unsigned parts) {
-  __shared__ float tile[kStripK][34];
+  __shared__ __align__(16) float tile[kStripK][34];      // rows of 34: stored to as pairs
   __shared__ __align__(16) float warp_max[8][32];
   __shared__ float part_max[32];
   sm100::trigger_dependent_launch();       // the GEMM's set-up may run under this grid
