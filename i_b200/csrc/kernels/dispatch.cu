@@ -427,12 +427,12 @@ int contract_with_chain(const float* a, const float* b, float* c, size_t batch, 
     const bool b_rows = !dots && m == 1 && b_kmajor != 0;     // C[b][j] = A[b][:] . B[b][j][:]
     constexpr size_t kMostLaunches = 64;
     // Operators run in the fold's last step where that saves a launch and lengthens one fold only a little: one
-    // batch entry, and rows few enough that the one lane a row that applies them is not the longer part (with
-    // a full-size operand, fused / apart in us: 4096 x 4096 14.5 / 16.5, 10000 x 200 8.3 / 10.4, 20000 x 2000
-    // 39.7 / 38.3, 200000 x 20 46.6 / 28.9; 8 entries of 1000 x 100 49 / 37).  Down the columns a thread has
-    // a column each.
+    // batch entry or two, and rows few enough that the one lane a row that applies them is not the longer part
+    // (with a full-size operand, fused / apart in us: 4096 x 4096 14.5 / 16.5, 10000 x 200 8.3 / 10.4, 20000 x
+    // 2000 39.7 / 38.3, 200000 x 20 46.6 / 28.9; two entries of 1000 x 1000 12.4 / 14.7, of 20000 x 100 16.5 /
+    // 12.5; eight of 1000 x 100 49 / 37).  Down the columns a thread has a column each.
     constexpr size_t kFusedRows = 12000;
-    const bool rows_fused = batch == 1 && n <= kFusedRows;
+    const bool rows_fused = batch <= 2 && n <= (batch == 1 ? kFusedRows : kFusedRows / 4);
     if (dots || ((a_rows || b_rows) && batch <= kMostLaunches)) {
       int rc = 0;
       if (dots) {
