@@ -26,6 +26,9 @@ HAVE_GPU = _have_gpu()
 
 
 def pytest_collection_modifyitems(config, items):
+    # The tests that run the reference's own scripts need copies of them, which only its checkout can give:
+    # last, so that a run that stops at the first failure has run everything else.
+    items.sort(key=lambda item: "test_gpu_reference_frontend" in item.nodeid)
     if HAVE_GPU:
         return
     skip = pytest.mark.skip(reason="no CUDA device")

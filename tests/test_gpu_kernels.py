@@ -1149,3 +1149,27 @@ def test_attention_divides_keys_where_the_arm_gains(lib, torch, precision, tol, 
         torch.cuda.synchronize()
         assert ((o.double() - want).abs().max() / want.abs().max()).item() <= tol
     assert launches[0] - launches[1] == (precision in divided)
+
+
+@pytest.mark.parametrize("nq,nk,d", [(3, 700, 32), (1, 9000, 128), (12, 100, 64), (8, 33, 20)])
+def test_attention_direct_fp32_special_values(lib, torch, nq, nk, d):
+    # As the reference's chain has it: a key at -inf weighs nothing, a row of such keys alone, a score of +inf
+    # and a NaN give NaN, each in its own row or head only.  One head each; whole blocks of keys are masked.
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nk)
+    q, k, v = (torch.randn(6, n, d, device="cuda", generator=g) * 0.3 for n in (nq, nk, nk))
+    q[:, :, 0] = 1.0
+    k[1, : nk // 2, 0] = -float("inf")                    # half masked: the first blocks have no finite score
+    k[2, :, 0] = -float("inf")
+    k[3, nk - 1, 0] = float("inf")
+    q[4, nq - 1, 1] = float("nan")
+    v[5, nk // 3, 2] = float("nan")
+    ws_bytes = lib.ib_attention_workspace_bytes(6, nq, nk, d, d, 0, FP32)
+    ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device="cuda")
+    o = torch.zeros(6, nq, d, device="cuda")
+    ok(lib, lib.ib_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 6, nq, nk, d, d, 0, FP32, 0,
+                             ws.data_ptr(), ws_bytes, None))
+    want = torch.softmax(q.double() @ k.double().transpose(1, 2), -1) @ v.double()
+    assert torch.equal(torch.isnan(o), torch.isnan(want))
+    assert torch.isnan(want[2]).all() and torch.isnan(want[3]).all() and not torch.isnan(want[:2]).any()
+    assert torch.nan_to_num(o.double() - want).abs().max().item() <= 1e-5 * torch.nan_to_num(want).abs().max().item()
