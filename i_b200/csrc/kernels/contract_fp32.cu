@@ -18,8 +18,8 @@
 // (fp32_copies).
 //
 // Measured on B200, against 64 x 64 tiles of 4 x 4 results with 4-byte shared-memory reads: 1024 x
-// 1000 x 1001 145 -> 62 us, 2048 x 2048 x 512 105 us (41 TFLOP/s; the FMA pipe is 66-69 % busy, held
-// by the waits between a quad's packing and its use), 32 x 32 x 2048 226 -> 10 us.
+// 1000 x 1001 145 -> 62 us, 2048 x 2048 x 512 105 us (41 TFLOP/s), 32 x 32 x 2048 226 -> 10 us.  At 1024 x 1000 x
+// 1001 the FMA pipe is busy 62 % of the time; stalls: the pipe itself, and waits between a quad's packing and its use.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

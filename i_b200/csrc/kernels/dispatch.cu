@@ -64,8 +64,8 @@ bool wants_tensor(int precision, double flop) {
   return true;
 }
 
-// AUTO takes the fp16 arm for a contraction only where its two conversion passes (each operand
-// read twice and written once at half size) are paid back by the faster MMAs: both output extents
+// AUTO takes the fp16 arm for a contraction only where the conversion of its operands (each read
+// once and written at half size, in one launch) is paid back by the faster MMAs: both output extents
 // large against the operand sizes and a deep contraction.  Measured on B200: 8192 x 8192 x 4096 runs
 // 1.58x faster than the TF32 arm, 8192 x 8192 x 512 and 16384 x 128 x 16384 slower.
 bool contract_prefers_f16(size_t m, size_t n, size_t k) {
